@@ -181,14 +181,11 @@ __device__ __forceinline__ void route(const DevJob &J, int node) {
 // the mixed kernel already solved are recomputed, so every result is the
 // FP64 one).
 //
-// The break-even points, measured: a 32-row FP32 attempt costs about 0.42 of
-// the exact 32-row solve (23.2 vs 54.8 ms over the SK 256x256x64 job), so
-// attempts pay above 42 % successes (keep 0.5, abandon above 60 % routed);
-// a 64-row attempt costs about 0.82 of the exact 64-row solve (the median
-// over serving jobs of 38-60 neighbours with nothing routed), so they pay
-// only above about 82 % successes (keep 0.85, abandon above 15 % routed).
+// The break-even point, measured: a 64-row attempt costs about 0.82 of the
+// exact 64-row solve (the median over serving jobs of 38-60 neighbours with
+// nothing routed), so they pay only above about 82 % successes (keep 0.85,
+// abandon above 15 % routed).
 constexpr int ABANDON_MIN = 4096;
-constexpr float ROUTE_KEEP32 = 0.5f, ABANDON_FRACTION32 = 0.6f;
 constexpr float ROUTE_KEEP64 = 0.85f, ABANDON_FRACTION64 = 0.15f;
 
 struct AttemptTally {

@@ -29,7 +29,7 @@
 namespace hpgl_b200 {
 
 // jobs of at most this many neighbours take the exact path when mixed is asked for
-constexpr int MIXED_MIN_NEIGHBOURS = 12;
+constexpr int MIXED_MIN_NEIGHBOURS = 32;
 
 #define CUDA_CHECK(expr)                                                                              \
     do {                                                                                              \
@@ -108,7 +108,8 @@ struct Arena {
 
 struct JobState {
     hpgl_b200_job_t job;
-    int precision;
+    int precision;   // as asked for (launch settings)
+    bool mixed;      // run the FP32 + refinement path
     long long size;
     int K;
     bool per_category;
@@ -259,11 +260,11 @@ static void prepare(JobState &S, const hpgl_b200_job_t &job, const hpgl_b200_res
         throw HpglError{HPGL_E_INVALID, e.what()};
     }
     // Up to MIXED_MIN_NEIGHBOURS neighbours the exact solve is the faster one
-    // (its factorisation stops at n, the FP32 sweep always runs 32 rows: the
-    // mixed solve takes 1.25-1.33x the exact one at 8-9 neighbours and 0.69x
-    // at 19), so a mixed request takes the exact path, whose results are the
-    // FP64 ones.
-    if (S.precision == HPGL_PRECISION_MIXED && S.nmax_all <= MIXED_MIN_NEIGHBOURS) S.precision = HPGL_PRECISION_FP64;
+    // (SK 256x256x64, 32 neighbours: 17.9 ms, an FP32 inverse with FP64
+    // refinement 22.5 ms; IK 200x200x100, 24: 9.2 and 20.7 ms), so a mixed
+    // request takes it and gets the FP64 results; its launch setting stays the
+    // mixed one's.
+    S.mixed = S.precision == HPGL_PRECISION_MIXED && S.nmax_all > MIXED_MIN_NEIGHBOURS;
     if (S.cok) {
         // cross covariance models (simple_cokriging_markI.cpp:140-181); the
         // means are mean_t (float) in the reference
@@ -442,6 +443,13 @@ static void upload_rest(JobState &S, cudaStream_t s) {
         d.syx = d.sx * (2 * P.B[1] + 1);
         d.center = P.B[2] * d.syx + P.B[1] * d.sx + P.B[0];
         d.truncated = P.truncated ? 1 : 0;
+        {
+            // offsets reach the radii (template) or 2 r - 1 (clusterizer boxes)
+            const int n3[3] = {P.nx, P.ny, P.nz}, t3[3] = {d.Tx, d.Ty, d.Tz};
+            int reach[3];
+            for (int a = 0; a < 3; ++a) reach[a] = (int)std::min<long long>(n3[a] - 1, 4LL * P.radii[a]);
+            d.pk = OffsetPack(reach, t3);
+        }
         d.c0 = P.c0;
         d.bucket_start = at<int>(S, g.o_bstart);
         d.bucket_nodes = at<int>(S, g.o_bnodes);
@@ -551,7 +559,7 @@ static void device_pass(JobState &S, cudaStream_t s, PassTiming *pt,
         const LaunchTuning tune64 = tuning_get(tuning_family(g.plan.nmax), HPGL_PRECISION_FP64);
         if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->search0, s));
         CUDA_CHECK(cudaMemsetAsync(J.nbcount, 0, (size_t)S.size * sizeof(int), s));
-        if (S.precision == HPGL_PRECISION_MIXED) CUDA_CHECK(cudaMemsetAsync(J.routed, 0, (size_t)S.size, s));
+        if (S.mixed) CUDA_CHECK(cudaMemsetAsync(J.routed, 0, (size_t)S.size, s));
         launch_build_bits(J, g.dp, at<uint32_t>(S, g.o_bits), s);
         ++launches;
         if (S.cok) {
@@ -581,15 +589,15 @@ static void device_pass(JobState &S, cudaStream_t s, PassTiming *pt,
         }
         if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top0, s));
         if (tune.schedule == SCHED_FUSED) {
-            if (g.plan.nmax <= 32) launch_fused32(J, g.dp, S.precision, s, tune.blocks_per_sm);
-            else launch_fused64(J, g.dp, S.precision, s, tune.blocks_per_sm);
+            if (g.plan.nmax <= 32) launch_fused32(J, g.dp, s, tune.blocks_per_sm);
+            else launch_fused64(J, g.dp, S.mixed, s, tune.blocks_per_sm);
         } else {
             CUDA_CHECK(cudaMemsetAsync(J.node_next, 0, sizeof(int), s));  // the mixed kernel's chunk counter
-            launch_solve(J, g.dp, S.precision, nullptr, s, tune.blocks_per_sm);
+            launch_solve(J, g.dp, S.mixed ? HPGL_PRECISION_MIXED : HPGL_PRECISION_FP64, nullptr, s, tune.blocks_per_sm);
         }
         ++launches;
         if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top1, s));
-        if (S.precision == HPGL_PRECISION_MIXED) {
+        if (S.mixed) {
             CUDA_CHECK(cudaMemsetAsync(J.node_next, 0, sizeof(int), s));  // an abandoned job's full FP64 pass
             launch_solve(J, g.dp, HPGL_PRECISION_FP64, J.routed, s, tune64.blocks_per_sm);
             ++launches;
@@ -597,7 +605,7 @@ static void device_pass(JobState &S, cudaStream_t s, PassTiming *pt,
         if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->resolve1, s));
         CUDA_CHECK(cudaGetLastError());
         if (after_group) after_group(g);
-        if (S.precision == HPGL_PRECISION_MIXED && gi + 1 < S.groups.size()) {
+        if (S.mixed && gi + 1 < S.groups.size()) {
             // the routed count and the job-level tally start over per group
             CUDA_CHECK(cudaMemsetAsync(&cnt->n_routed, 0, sizeof(int), s));
             CUDA_CHECK(cudaMemsetAsync(&cnt->n_attempt, 0, 3 * sizeof(int), s));
@@ -1018,13 +1026,13 @@ static void sgs_run(JobState &S, hpgl_b200_result_t &res, SyncContext &C, std::c
     res.rounds = hc.rounds;
 }
 
-static const char *top_kernel_name(int nmax, int precision, int schedule, const DevPlan &dp) {
+static const char *top_kernel_name(int nmax, bool mixed, int schedule) {
     if (schedule == SCHED_FUSED) {
-        if (nmax <= 32) return precision ? "k_fused32<1>" : "k_fused32<0>";
-        return precision ? "k_fused64<1>" : "k_fused64<0>";
+        if (nmax <= 32) return "k_fused32";
+        return mixed ? "k_fused64<1>" : "k_fused64<0>";
     }
-    if (nmax <= 32) return precision ? mixed32_kernel_name(dp) : "k_solve_exact32";
-    return precision ? "k_solve_mixed64" : "k_solve_exact64";
+    if (nmax <= 32) return "k_solve_tile";
+    return mixed ? "k_solve_mixed64" : "k_solve_exact64";
 }
 
 // The job's device pass captured once as a CUDA graph and replayed for every
@@ -1110,8 +1118,8 @@ void bench_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res, hpgl_b200_be
     bench.ms_resolve = resolve_sum / phase_runs;
     snprintf(bench.top_kernel, sizeof(bench.top_kernel), "%s",
              S.cok ? "k_cokriging"
-                   : top_kernel_name(S.nmax_all, S.precision,
-                                     tuning_get(tuning_family(S.nmax_all), S.precision).schedule, S.groups[0].dp));
+                   : top_kernel_name(S.nmax_all, S.mixed,
+                                     tuning_get(tuning_family(S.nmax_all), S.precision).schedule));
     bench.launches_per_iter = pt.launches;
     cudaEventDestroy(pt.search0);
     cudaEventDestroy(pt.top0);

@@ -318,7 +318,7 @@ void launch_solve(const DevJob &J, const DevPlan &P, int precision, const uint8_
                   int blocks_per_sm) {
     if (J.size <= 0) return;
     if (P.nmax <= 32) {
-        launch_solve32(J, P, precision, routed, s, blocks_per_sm);
+        if (!routed) launch_solve32(J, P, s, blocks_per_sm);  // nothing is ever routed
         return;
     }
     if (precision == 0 || routed) launch_solve64_exact(J, P, routed, s, blocks_per_sm);

@@ -3,6 +3,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "offset_pack.h"
+
 namespace hpgl_b200 {
 
 enum Status : int8_t { ST_SUCCESS = 0, ST_NO_NEIGHBOURS = 1, ST_SINGULAR = 2, ST_NOT_KRIGED = -1 };
@@ -29,6 +31,7 @@ struct DevPlan {
     int center;              // table index of offset 0
     int truncated;           // beyond T is the model's 0 (else a broken invariant)
     double c0;
+    OffsetPack pk;           // packed neighbour offsets and the range test on their differences
     // clusterizer
     const int *bucket_start;
     const int *bucket_nodes;
@@ -213,19 +216,18 @@ void launch_sis_round(const DevJob &J, const DevPlan &P0, const DevPlan *plans, 
                       int cur, cudaStream_t s);
 void launch_sis_try32(const DevJob &J, const DevPlan *plans, const SgsState &G, int cur, cudaStream_t s);
 void launch_sis_try64(const DevJob &J, const DevPlan *plans, const SgsState &G, int cur, cudaStream_t s);
-// solve32.cu: the mixed-precision kernel launch_solve32 runs for plan P
-const char *mixed32_kernel_name(const DevPlan &P);
-// solve32.cu: register-resident solves for max_neighbours <= 32
-void launch_solve32(const DevJob &J, const DevPlan &P, int precision, const uint8_t *routed, cudaStream_t s,
-                    int blocks_per_sm);
+// solve32.cu: solves for max_neighbours <= 32, exact FP64 for either precision
+// (every node; the FP64 solve of the tiled kernels is faster than an FP32 one
+// with refinement was)
+void launch_solve32(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm);
 // solve64.cu: solves for 33..64 neighbours (exact FP64; FP32 inverse + FP64
 // refinement, routing to `routed`)
 void launch_solve64_exact(const DevJob &J, const DevPlan &P, const uint8_t *routed, cudaStream_t s,
                           int blocks_per_sm);
 void launch_solve64_mixed(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm);
 // Fused template search + solve of every node (the clusterizer search runs
-// first); precision 0 exact FP64, 1 mixed.
-void launch_fused32(const DevJob &J, const DevPlan &P, int precision, cudaStream_t s, int blocks_per_sm);
+// first); precision 0 exact FP64, 1 mixed (33-64 neighbours).
+void launch_fused32(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm);
 void launch_fused64(const DevJob &J, const DevPlan &P, int precision, cudaStream_t s, int blocks_per_sm);
 
 }  // namespace hpgl_b200

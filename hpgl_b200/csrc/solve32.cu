@@ -1,24 +1,19 @@
-// Register-resident per-node solves for systems of at most 32 neighbours
-// (one warp per system, persistent over the grid's nodes).
+// Per-node solves for systems of at most 32 neighbours, FP64 in the
+// reference's exact operation order (my_kriging_weights.h:26-255 over LAPACK
+// DPOTF2 / DPOTRS).
 //
-//   k_solve_exact32  FP64 in the reference's exact operation order
-//                    (my_kriging_weights.h:26-255 over LAPACK DPOTF2/DPOTRS):
-//                    lane k holds column k of the system in registers; the
-//                    finished part of column j is broadcast through shared
-//                    memory as 16-byte pairs for the dot products of step j.
-//   k_solve_mixed32  FP32 Gauss-Jordan inverse of the (unit-diagonal scaled)
-//                    system, lane r holding row r, every solve a parallel
-//                    matrix-vector product; FP64 residuals against the exact
-//                    FP64 system refine the solution.  Systems whose FP32
-//                    pivots fall below 1e-3 (the FP64 factorisation cannot
-//                    fail above that), or whose refinement stalls, are routed
-//                    to the exact kernel.
-//
-// Both start from the same system: neighbour offsets from the search lists
-// and covariances gathered from the plan's table (my_kriging_weights.h:49-58,
-// 156-165), padded to 32x32 with the identity.
+//   k_solve_tile     (tile_solve.cuh) several systems a warp, persistent over
+//                    the grid's nodes: every kriging job's solve.
+//   exact_core       one system a warp, lane k holding column k in registers,
+//                    the finished part of column j broadcast through shared
+//                    memory as 16-byte pairs for the dot products of step j:
+//                    sequential simulation (a node's search and system in one
+//                    warp, one node at a time), the fused search + solve
+//                    kernel, and the jobs the tiled kernels do not take
+//                    (k_solve_exact32).
 #include "device_common.cuh"
 #include "search_common.cuh"
+#include "tile_solve.cuh"
 
 namespace hpgl_b200 {
 
@@ -26,18 +21,15 @@ namespace {
 
 constexpr int N32 = 32;
 constexpr int WARPS32 = 4;
-constexpr int MIXED_CHUNK = 32;  // at most this many nodes a warp takes from the counter at a time
-constexpr float MIXED_PIVOT_MIN = 1e-3f;  // on the unit-diagonal scaled system
-constexpr int MIXED_MAX_CORR = 4;
 
-// Per-warp shared memory; NA doubles of system storage (the exact path uses
-// columns of 34: NC * 34 for systems of at most NC neighbours).
+// Per-warp shared memory; NA doubles of system storage (columns of 34: NC *
+// 34 for systems of at most NC neighbours).
 template <int NA>
 struct SysSmemN {
-    double A[NA];           // exact: in-place factor (column k at k*34); mixed: full system (LD 32, msw)
+    double A[NA];           // in-place factor (column k at k*34)
     double vd[N32];         // double vector broadcast
     float vf[2][N32];       // float vector broadcast
-    float row[2][N32];      // mixed: pivot row broadcast (double buffered)
+    float row[2][N32];      // simulation: the neighbour list
     int4 nb[N32];           // neighbour offsets from the node (x, y, z, table offset)
 };
 using SysSmem = SysSmemN<N32 * 34>;
@@ -46,18 +38,7 @@ using SysSmem = SysSmemN<N32 * 34>;
 constexpr int N16 = 16;
 using SysSmem16 = SysSmemN<N16 * 34>;
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
-    return v;
-}
-__device__ __forceinline__ double warp_max(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(FULL_MASK, v, o));
-    return v;
-}
-
-// Per-node prologue shared by both kernels.  Returns n (neighbour count) and
+// Per-node prologue.  Returns n (neighbour count) and
 // fills the lane's neighbour data; the system itself is built separately.
 struct NodeData {
     int n;
@@ -101,46 +82,6 @@ __device__ __forceinline__ NodeData load_node(const DevJob &J, const DevPlan &P,
     S.nb[lane] = make_int4(ox, oy, oz, d.lin);
     __syncwarp();
     return d;
-}
-
-// Position of A(i, j) in the mixed kernel's FP64 system: column j at j*32,
-// row i XOR-swizzled by j/4 within it.  A lane reading its row (the FP64
-// residuals, lane = row) and the lanes reading 8x4 tiles (the FP32 copy,
-// rows 8 (lane/8) .. +7, columns 4 (lane%8) .. +3) both hit every
-// shared-memory bank at most twice per 32 doubles, the minimum; the build's
-// stores along the cyclic diagonals (l, l+d) and (l+d, l) take 86
-// wavefronts a system against 62 at best (128 with a column stride of 33).
-__device__ __forceinline__ int msw(int i, int j) { return j * 32 + (i ^ (j >> 2)); }
-
-// The full symmetric system into S.A (column k at k*32, msw): the entries
-// A(i,k) = C(x_i - x_k) (my_kriging_weights.h:49-58, 156-165; the tables
-// are exactly symmetric, C(v) = C(-v) bit for bit, so either orientation
-// gives the reference's value); diagonal C(0); the identity beyond n.
-// Lane l takes the pairs (l, l+d mod 32), d = 1..16 (d = 16 on lanes 0-15
-// only): every off-diagonal pair once, all 16 gathers of a lane in flight
-// together, and the zero padding written by the same stores.
-__device__ __forceinline__ void build_full32(const DevJob &J, const DevPlan &P, SysSmem &S, int n, int lane) {
-    const int4 a = S.nb[lane];
-    double v[16];
-#pragma unroll
-    for (int d = 1; d <= 16; ++d) {
-        const int k = (lane + d) & 31;
-        v[d - 1] = 0.0;
-        if (lane < n && k < n && (d < 16 || lane < 16)) {
-            const int4 b = S.nb[k];
-            v[d - 1] = cov_lin(P, a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w, J.err);
-        }
-    }
-#pragma unroll
-    for (int d = 1; d <= 16; ++d) {
-        const int k = (lane + d) & 31;
-        if (d < 16 || lane < 16) {
-            S.A[msw(lane, k)] = v[d - 1];
-            S.A[msw(k, lane)] = v[d - 1];
-        }
-    }
-    S.A[msw(lane, lane)] = lane < n ? __ldg(P.table + P.center) : 1.0;
-    __syncwarp();
 }
 
 // init + t_0 + t_1 + ... + t_{n-1} in that order, t_i = `term` of lane i,
@@ -264,7 +205,6 @@ __device__ __forceinline__ bool copy_informed(const DevJob &J, const NodeFetch &
 }
 
 // ---------------------------------------------------------------------------
-// Exact FP64 path.
 
 // IEEE square root and reciprocal (one lane per factorisation step).
 __device__ __noinline__ double dsqrt_rn(double a) { return __dsqrt_rn(a); }
@@ -428,331 +368,36 @@ __device__ __forceinline__ bool exact32_node(const DevJob &J, const DevPlan &P, 
     return true;
 }
 
-// routed: per-node flags of the mixed pass -- the flagged nodes are solved,
-// 32 flags read at a time and taken in node order (every node once the job
-// was abandoned); null: every node.
-__global__ void __launch_bounds__(WARPS32 * 32) k_solve_exact32(DevJob J, DevPlan P, const uint8_t *routed) {
+// Every node, for the jobs the tiled kernels do not take (tile_takes).
+// Warps take up to 32 consecutive nodes at a time from the per-job counter.
+__global__ void __launch_bounds__(WARPS32 * 32) k_solve_exact32(DevJob J, DevPlan P) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     SysSmem &S = reinterpret_cast<SysSmem *>(dyn_smem)[warp];
-    const long long stride = (long long)gridDim.x * WARPS32;
     unsigned long long solved = 0;
-    long long it = (long long)blockIdx.x * WARPS32 + warp;
-    if (routed && !*J.abandon) {
-        for (long long base = it * 32; base < J.size; base += stride * 32) {
-            const long long i = base + lane;
-            unsigned m = __ballot_sync(FULL_MASK, i < J.size && routed[i]);
-            while (m) {
-                const int k = __ffs(m) - 1;
-                m &= m - 1;
-                const NodeFetch f = fetch_node(J, P, (int)(base + k), lane);
-                solved += exact32_node(J, P, S, f, lane);
-                __syncwarp();
-            }
-        }
-    } else {
-        // warps take up to MIXED_CHUNK consecutive nodes at a time from the per-job
-        // counter, as the mixed kernel
-        const int csize = chunk_nodes(J, MIXED_CHUNK, WARPS32);
-        int chunk = 0;
-        if (lane == 0) chunk = atomicAdd(J.node_next, csize);
-        chunk = __shfl_sync(FULL_MASK, chunk, 0);
-        it = chunk;
-        NodeFetch cur = fetch_node(J, P, it < J.size ? (int)it : -1, lane);
-        while (it < J.size) {
-            long long nx = it + 1;
-            int nchunk = chunk;
-            if (nx == (long long)chunk + csize) {
-                int c = 0;
-                if (lane == 0) c = atomicAdd(J.node_next, csize);
-                nchunk = __shfl_sync(FULL_MASK, c, 0);
-                nx = nchunk;
-            }
-            const NodeFetch next = fetch_node(J, P, nx < J.size ? (int)nx : -1, lane);
-            solved += exact32_node(J, P, S, cur, lane);
-            __syncwarp();
-            cur = next;
-            it = nx;
-            chunk = nchunk;
-        }
-    }
-    if (lane == 0 && solved) atomicAdd(J.n_fp64, solved);
-}
-
-// ---------------------------------------------------------------------------
-// Mixed path.
-
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-
-// The FP32 inverse is held in 8x4 tiles: lane l owns rows 8 (l/8) .. +7 and
-// columns 4 (l%8) .. +3, t[r][h] = (M(row r, col 2h), M(row r, col 2h+1)).
-// Per sweep step a lane needs the pivot row's 4 values at its columns and 8
-// at its rows (the pivot column, by symmetry): three 16-byte broadcast reads
-// and one store by the 8 lanes of the pivot row, half the shared-memory
-// traffic of a lane holding a whole row.
-struct Tile {
-    float2 t[8][2];
-};
-
-// y = (T - 2 I) v for v given row by row (v of row `lane`); returns y of row
-// `lane`.
-// Each lane forms its columns' partial sums over its rows (M is symmetric),
-// the four lanes of a column group add them up while scattering the four
-// columns among themselves (lane (g, c) ends with column 4c + g), and one
-// shuffle brings each row its value.
-__device__ __forceinline__ float apply_inverse(const Tile &T, float v, float *buf, int lane) {
-    buf[lane] = v;
-    __syncwarp();
-    const int rg = lane >> 3;
-    const float4 v0 = *reinterpret_cast<const float4 *>(buf + 8 * rg);
-    const float4 v1 = *reinterpret_cast<const float4 *>(buf + 8 * rg + 4);
-    const float vr[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-    float2 a01 = f2(0.f, 0.f), a23 = f2(0.f, 0.f);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        a01 = __ffma2_rn(T.t[r][0], f2(vr[r], vr[r]), a01);
-        a23 = __ffma2_rn(T.t[r][1], f2(vr[r], vr[r]), a23);
-    }
-    __syncwarp();
-    const bool hi2 = (rg & 2) != 0, hi1 = (rg & 1) != 0;
-    float2 keep = hi2 ? a23 : a01;
-    const float2 send = hi2 ? a01 : a23;
-    keep.x += __shfl_xor_sync(FULL_MASK, send.x, 16);
-    keep.y += __shfl_xor_sync(FULL_MASK, send.y, 16);
-    float k = hi1 ? keep.y : keep.x;
-    k += __shfl_xor_sync(FULL_MASK, hi1 ? keep.x : keep.y, 8);
-    // the sweep leaves +2 on the diagonal
-    return __shfl_sync(FULL_MASK, k, 8 * (lane & 3) + (lane >> 2)) - 2.f * v;
-}
-
-// r = b - A x in FP64 (row `lane`; S.A holds the full symmetric system, msw).
-template <typename SM>
-__device__ __forceinline__ double residual(const SM &S, double *vd, double x, double b, int lane) {
-    vd[lane] = x;
-    __syncwarp();
-    // four independent accumulation chains (the dot product's order is free
-    // on the refinement path)
-    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-    const double2 *x2 = reinterpret_cast<const double2 *>(vd);
-#pragma unroll
-    for (int q = 0; q < N32 / 4; ++q) {
-        const double2 u = x2[2 * q], w = x2[2 * q + 1];
-        acc0 = fma(S.A[msw(lane, 4 * q)], u.x, acc0);
-        acc1 = fma(S.A[msw(lane, 4 * q + 1)], u.y, acc1);
-        acc2 = fma(S.A[msw(lane, 4 * q + 2)], w.x, acc2);
-        acc3 = fma(S.A[msw(lane, 4 * q + 3)], w.y, acc3);
-    }
-    __syncwarp();
-    return b - ((acc0 + acc1) + (acc2 + acc3));
-}
-
-// The kriging variance of a refined solution, c0 - b.w (ordinary kriging:
-// c0 - b.w - w_{n-1}, my_kriging_weights.h:246), accurate to second order in
-// the solution's error.  With x the accepted solution and r = b - A x its
-// FP64 residual (A symmetric, A x* = b): b.x* = b.x + x*.r, taken as
-// b.x + x.r, whose error (x - x*).r is the product of two tiny quantities;
-// the same holds for the ordinary-kriging sums b.xb*, 1.xa*, 1.xb*
-// (A xb* = 1, its residual rb), from which mu and w_{n-1} are formed.
-// Where the variance is a small difference of c0 and b.w (nodes next to or
-// on informed cells), the plain sum would carry the refinement's relative
-// error of w (up to about 1e-13) straight into it.  One more residual per
-// right-hand side, only when variances are asked for.
-template <typename SM>
-__device__ __forceinline__ double residual_corrected_variance(const SM &S, double c0, double b, double ba,
-                                                              double bb, bool ordinary, int n, double xa,
-                                                              double xb, int lane) {
-    const double ra = residual(S, const_cast<double *>(S.vd), xa, ba, lane);
-    const double bxa = warp_sum(b * xa + xa * ra);
-    if (!ordinary) return c0 - bxa;
-    const double rb = residual(S, const_cast<double *>(S.vd), xb, bb, lane);
-    const double bxb = warp_sum(b * xb + xa * rb);
-    const double oxa = warp_sum(xa + xb * ra);
-    const double oxb = warp_sum(xb + xb * rb);
-    const double mu = (oxa - 1.0) / oxb;
-    const double wl = __shfl_sync(FULL_MASK, xa - mu * xb, n - 1);
-    return c0 - (bxa - mu * bxb) - wl;
-}
-
-// One node of the mixed path (FP32 inverse + FP64 refinement); systems that
-// do not qualify are appended to J.routed.  skip: a system is appended to
-// J.routed at once, without the FP32 attempt.  Returns -1 when the node
-// needs no system, 0 when it was solved here, 1 when routed.
-// STEPS: the sweep's pivots, at least the job's largest neighbour count (a
-// multiple of 8): rows from n on are identity padding, decoupled from the
-// live block, with zero right-hand sides, so their solutions stay zero
-// whether or not their pivots are swept; a job of at most 24 neighbours
-// sweeps 24 pivots, and the steps stay fully unrolled.
-template <int STEPS = N32>
-__device__ __forceinline__ int mixed32_node(const DevJob &J, const DevPlan &P, SysSmem &S, const NodeFetch &cur,
-                                            int lane, bool skip = false) {
-    const bool ordinary = J.kind == 0;
-    const double inv_c0 = 1.0 / P.c0;
-    const int node = cur.node;
-    if (copy_informed(J, cur, lane)) return -1;
-    if (skip && cur.n > 0) {
-        if (lane == 0) route(J, node);
-        __syncwarp();
-        return 1;
-    }
-    const NodeData d = load_node(J, P, S, cur, lane);
-    if (d.n <= 0) {
-        write_outputs(J, P, S, node, lane, d, ST_NO_NEIGHBOURS, 0.0, -1.0);
-        return -1;
-    }
-    const int n = d.n;
-    build_full32(J, P, S, n, lane);
-    // The lane's tile of the unit-diagonal system A / C(0) (identity padding).
-    const int rg = lane >> 3, cg = lane & 7;
-    Tile T;
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            T.t[r][h] = f2((float)(S.A[msw(8 * rg + r, 4 * cg + 2 * h)] * inv_c0),
-                           (float)(S.A[msw(8 * rg + r, 4 * cg + 2 * h + 1)] * inv_c0));
-    // Symmetric Gauss-Jordan sweeps (the sweep operator): the matrix stays
-    // symmetric, so row p is column p; the lanes holding row p publish it,
-    // every lane reads it at its columns (the update's right factor) and at
-    // its rows (its rows' multipliers).  The pivot's own entry of the right
-    // factor is taken as piv - 1, which turns the same fused update into the
-    // swept column p (m_rp / piv) on every other row and leaves 2 - 1/piv
-    // in place of -1/piv on the pivot itself; a swept diagonal entry is never
-    // read again, so after all sweeps T holds -(A/C(0))^-1 + 2 I and the
-    // products subtract the 2 v (apply_inverse).
-    bool low = false;
-#pragma unroll
-    for (int p = 0; p < STEPS; ++p) {
-        float *rb = S.row[p & 1];
-        const int rgp = p >> 3, rp = p & 7, cgp = p >> 2, cp = p & 3;
-        const bool prow = rg == rgp;
-        if (prow)
-            *reinterpret_cast<float4 *>(rb + 4 * cg) =
-                make_float4(T.t[rp][0].x, T.t[rp][0].y, T.t[rp][1].x, T.t[rp][1].y);
-        __syncwarp();
-        float4 cv = *reinterpret_cast<const float4 *>(rb + 4 * cg);
-        const float4 r0 = *reinterpret_cast<const float4 *>(rb + 8 * rg);
-        const float4 r1 = *reinterpret_cast<const float4 *>(rb + 8 * rg + 4);
-        const float piv = rb[p];
-        low |= !(piv > MIXED_PIVOT_MIN);
-        const float dinv = __fdividef(1.f, piv);  // approximate: the refinement absorbs it
-        if (cg == cgp) {
-            if (cp == 0) cv.x = piv - 1.f;
-            else if (cp == 1) cv.y = piv - 1.f;
-            else if (cp == 2) cv.z = piv - 1.f;
-            else cv.w = piv - 1.f;
-        }
-        const float rv[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-        const float2 nd = f2(-dinv, -dinv);
-        // the pivot row's multiplier is (m_pp - 1) / piv
-        const float dp = prow ? dinv : 0.f;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const float2 ng = __ffma2_rn(f2(rv[r], rv[r]), nd, r == rp ? f2(dp, dp) : f2(0.f, 0.f));
-            T.t[r][0] = __ffma2_rn(ng, f2(cv.x, cv.y), T.t[r][0]);
-            T.t[r][1] = __ffma2_rn(ng, f2(cv.z, cv.w), T.t[r][1]);
-        }
-        __syncwarp();
-    }
-    if (__any_sync(FULL_MASK, low)) {
-        if (lane == 0) route(J, node);
-        __syncwarp();
-        return 1;
-    }
-    // A^-1 v = -(M v) / C(0); solutions for b (and the ones vector for OK)
-    // refined with FP64 residuals.
-    const double sc = -inv_c0;
-    double xa = (double)apply_inverse(T, (float)d.b, S.vf[0], lane) * sc;
-    double xb = ordinary ? (double)apply_inverse(T, lane < n ? 1.f : 0.f, S.vf[1], lane) * sc : 0.0;
-    const double ba = d.b, bb = lane < n ? 1.0 : 0.0;
-    RefineGate gate;
-    bool converged = false;
-    for (int corr = 0; corr < MIXED_MAX_CORR; ++corr) {
-        const double ra = residual(S, S.vd, xa, ba, lane);
-        const double da = (double)apply_inverse(T, (float)ra, S.vf[0], lane) * sc;
-        xa += da;
-        double dmax = fabs(da), xmax = fabs(xa);
-        if (ordinary) {
-            const double rbv = residual(S, S.vd, xb, bb, lane);
-            const double db = (double)apply_inverse(T, (float)rbv, S.vf[1], lane) * sc;
-            xb += db;
-            dmax = fmax(dmax, fabs(db));
-            xmax = fmax(xmax, fabs(xb));
-        }
-        const int decision = gate.step(warp_max(dmax), warp_max(xmax));
-        if (decision != 0) {
-            converged = decision > 0;
-            break;
-        }
-    }
-    if (!converged) {
-        if (lane == 0) route(J, node);
-        __syncwarp();
-        return 1;
-    }
-    if (lane >= n) {
-        xa = 0.0;
-        xb = 0.0;
-    }
-    double w;
-    if (ordinary) {
-        const double mu = (warp_sum(xa) - 1.0) / warp_sum(xb);
-        w = xa - mu * xb;
-    } else {
-        w = xa;
-    }
-    double variance = -1.0;
-    if (J.variance) variance = residual_corrected_variance(S, P.c0, d.b, ba, bb, ordinary, n, xa, xb, lane);
-    write_outputs(J, P, S, node, lane, d, ST_SUCCESS, w, variance);
-    __syncwarp();
-    return 0;
-}
-
-template <int STEPS>
-__device__ __forceinline__ void mixed32_warps(const DevJob &J, const DevPlan &P) {
-    extern __shared__ __align__(16) unsigned char dyn_smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    SysSmem &S = reinterpret_cast<SysSmem *>(dyn_smem)[warp];
-    // Warps take MIXED_CHUNK consecutive nodes at a time from a per-job
-    // counter (the next chunk is taken while the current chunk's last node is
-    // solved), so none waits on a fixed share at the end.  The routing guess
-    // starts afresh with every chunk: its choices depend on the chunk's nodes
-    // only, whichever warp takes it.
+    const int csize = chunk_nodes(J, 32, WARPS32);
     int chunk = 0;
-    if (lane == 0) chunk = atomicAdd(J.node_next, MIXED_CHUNK);
+    if (lane == 0) chunk = atomicAdd(J.node_next, csize);
     chunk = __shfl_sync(FULL_MASK, chunk, 0);
     long long it = chunk;
-    NodeFetch next = fetch_node(J, P, it < J.size ? (int)it : -1, lane);
-    RouteGuess guess(ROUTE_KEEP32);
-    AttemptTally tally(ABANDON_FRACTION32);
+    NodeFetch cur = fetch_node(J, P, it < J.size ? (int)it : -1, lane);
     while (it < J.size) {
-        const NodeFetch cur = next;
-        if (it == chunk) guess = RouteGuess(ROUTE_KEEP32);
-        long long nit = it + 1;
+        long long nx = it + 1;
         int nchunk = chunk;
-        if (nit == (long long)chunk + MIXED_CHUNK) {
+        if (nx == (long long)chunk + csize) {
             int c = 0;
-            if (lane == 0) c = atomicAdd(J.node_next, MIXED_CHUNK);
+            if (lane == 0) c = atomicAdd(J.node_next, csize);
             nchunk = __shfl_sync(FULL_MASK, c, 0);
-            nit = nchunk;
+            nx = nchunk;
         }
-        next = fetch_node(J, P, nit < J.size ? (int)nit : -1, lane);
-        const bool attempt = guess.attempt();
-        const int outcome = mixed32_node<STEPS>(J, P, S, cur, lane, !attempt);
-        guess.record(attempt, outcome);
+        const NodeFetch next = fetch_node(J, P, nx < J.size ? (int)nx : -1, lane);
+        solved += exact32_node(J, P, S, cur, lane);
         __syncwarp();
-        if (tally.step(J, attempt, outcome, lane)) break;
-        it = nit;
+        cur = next;
+        it = nx;
         chunk = nchunk;
     }
-}
-
-__global__ void __launch_bounds__(WARPS32 * 32) k_solve_mixed32(DevJob J, DevPlan P) { mixed32_warps<N32>(J, P); }
-
-// jobs of at most 16 or 24 neighbours: the sweep stops there (held to 4
-// blocks a SM, the 128 registers the full sweep compiles to by itself)
-template <int STEPS>
-__global__ void __launch_bounds__(WARPS32 * 32, 4) k_solve_mixed32_short(DevJob J, DevPlan P) {
-    mixed32_warps<STEPS>(J, P);
+    if (lane == 0 && solved) atomicAdd(J.n_fp64, solved);
 }
 
 // Fused search + solve: each warp takes 32-node x-segments, runs the template
@@ -761,7 +406,6 @@ __global__ void __launch_bounds__(WARPS32 * 32, 4) k_solve_mixed32_short(DevJob 
 // nodes' lists come from the clusterizer search launched before.  Warps in
 // the search phase (memory latency) and in the solve phase (FP pipes)
 // overlap on every SM.
-template <int MODE>
 __global__ void __launch_bounds__(WARPS32 * 32) k_fused32(DevJob J, DevPlan P) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     __shared__ int delta_sm[WARPS32][32];
@@ -779,12 +423,11 @@ __global__ void __launch_bounds__(WARPS32 * 32) k_fused32(DevJob J, DevPlan P) {
         for (int b = 0; b < cnt; ++b) {
             const NodeFetch cur = next;
             next = fetch_node(J, P, b + 1 < cnt ? base + b + 1 : -1, lane);
-            if (MODE == 0) solved += exact32_node(J, P, S, cur, lane);
-            else mixed32_node(J, P, S, cur, lane);
+            solved += exact32_node(J, P, S, cur, lane);
             __syncwarp();
         }
     }
-    if (MODE == 0 && lane == 0 && solved) atomicAdd(J.n_fp64, solved);
+    if (lane == 0 && solved) atomicAdd(J.n_fp64, solved);
 }
 
 constexpr size_t SMEM32 = sizeof(SysSmem) * WARPS32;
@@ -979,39 +622,48 @@ void launch_sis_try32(const DevJob &J, const DevPlan *plans, const SgsState &G, 
     k_sis_try32<N32><<<(unsigned)g, WARPS32 * 32, SMEM32, s>>>(J, plans, G, cur);
 }
 
-void launch_fused32(const DevJob &J, const DevPlan &P, int precision, cudaStream_t s, int blocks_per_sm) {
+void launch_fused32(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
     const long long segs = (long long)P.nseg * J.ny * J.nz;
     if (segs <= 0) return;
     const int threads = WARPS32 * 32;
-    if (precision == 0) {
-        const long long g = persistent_grid((const void *)k_fused32<0>, threads, SMEM32, blocks_per_sm,
-                                            (segs + WARPS32 - 1) / WARPS32);
-        k_fused32<0><<<(unsigned)g, threads, SMEM32, s>>>(J, P);
-    } else {
-        const long long g = persistent_grid((const void *)k_fused32<1>, threads, SMEM32, blocks_per_sm,
-                                            (segs + WARPS32 - 1) / WARPS32);
-        k_fused32<1><<<(unsigned)g, threads, SMEM32, s>>>(J, P);
-    }
+    const long long g =
+        persistent_grid((const void *)k_fused32, threads, SMEM32, blocks_per_sm, (segs + WARPS32 - 1) / WARPS32);
+    k_fused32<<<(unsigned)g, threads, SMEM32, s>>>(J, P);
 }
 
-const char *mixed32_kernel_name(const DevPlan &P) { return P.nmax <= 24 ? "k_solve_mixed32_short" : "k_solve_mixed32"; }
-
-void launch_solve32(const DevJob &J, const DevPlan &P, int precision, const uint8_t *routed, cudaStream_t s,
-                    int blocks_per_sm) {
-    const int threads = WARPS32 * 32;
-    const long long units = (J.size + WARPS32 - 1) / WARPS32;
-    if (precision == 0 || routed) {
-        const long long g = persistent_grid((const void *)k_solve_exact32, threads, SMEM32, blocks_per_sm, units);
-        k_solve_exact32<<<(unsigned)g, threads, SMEM32, s>>>(J, P, routed);
+// The tile of a job's systems by its largest neighbour count.  Fewer lanes a
+// system share each step's pivot chain among more systems and read fewer
+// shared-memory words per product, until the lane's accumulators no longer
+// fit the registers: 4 lanes (8 systems a warp) up to 24 neighbours, 8 above;
+// the panel (row blocks whose sums are kept open together) is the widest
+// that does not spill.  Solve of the IK 200x200x100 job (4.0 M systems) with
+// the neighbour count set, in ms:
+//   8: 1.09   12: 2.03   16: 3.11   20: 7.1   24: 9.2   28: 14.7
+// against 39.7 at 24 with one column per lane and one system a warp; SK
+// 256x256x64 (4.15 M systems, 32 neighbours) 17.9 against 53.2, OK 20.2
+// against 57.1.  The neighbouring tiles, measured on earlier builds: 12 as 8
+// lanes 3.5; 16 as 8 lanes 5.2; 20 as 8 lanes 8.4; 24 as 8 lanes 9.6; 32 as
+// 16 lanes 21.0 where 8 lanes took 19.2.
+void launch_solve32(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
+    const int b = blocks_per_sm;
+    if (!tile_takes(P)) {
+        const long long g = persistent_grid((const void *)k_solve_exact32, WARPS32 * 32, SMEM32, b,
+                                            (J.size + WARPS32 - 1) / WARPS32);
+        k_solve_exact32<<<(unsigned)g, WARPS32 * 32, SMEM32, s>>>(J, P);
+    } else if (P.nmax <= 8) {
+        launch_tile<TileGeom<8, 4, 1, 2, 10>, 4, 5>(J, P, s, b);
+    } else if (P.nmax <= 12) {
+        launch_tile<TileGeom<12, 4, 1, 4, 10>, 4, 4>(J, P, s, b);
+    } else if (P.nmax <= 16) {
+        launch_tile<TileGeom<16, 4, 1, 2, 10>, 4, 3>(J, P, s, b);
+    } else if (P.nmax <= 20) {
+        launch_tile<TileGeom<20, 4, 1, 2, 10>, 4, 2>(J, P, s, b);
+    } else if (P.nmax <= 24) {
+        launch_tile<TileGeom<24, 4, 1, 2, 10>, 4, 2>(J, P, s, b);
+    } else if (P.nmax <= 28) {
+        launch_tile<TileGeom<28, 4, 2, 4, 8>, 4, 2>(J, P, s, b);
     } else {
-        // the sweep's length: the job's largest neighbour count rounded up to 8
-        const int steps = P.nmax <= 16 ? 16 : (P.nmax <= 24 ? 24 : 32);
-        const void *k = steps == 16 ? (const void *)k_solve_mixed32_short<16>
-                                    : (steps == 24 ? (const void *)k_solve_mixed32_short<24> : (const void *)k_solve_mixed32);
-        const long long g = persistent_grid(k, threads, SMEM32, blocks_per_sm, units);
-        if (steps == 16) k_solve_mixed32_short<16><<<(unsigned)g, threads, SMEM32, s>>>(J, P);
-        else if (steps == 24) k_solve_mixed32_short<24><<<(unsigned)g, threads, SMEM32, s>>>(J, P);
-        else k_solve_mixed32<<<(unsigned)g, threads, SMEM32, s>>>(J, P);
+        launch_tile<TileGeom<32, 4, 2, 4, 8>, 4, 2>(J, P, s, b);
     }
 }
 

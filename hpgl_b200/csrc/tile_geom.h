@@ -1,0 +1,68 @@
+// Lane tile and shared-memory layout of a small system (tile_solve.cuh):
+// plain constants, compiled for host and device.
+#pragma once
+
+#ifdef __CUDACC__
+#define HPGL_TILE_HD __host__ __device__
+#else
+#define HPGL_TILE_HD
+#endif
+
+namespace hpgl_b200 {
+
+// Layout of an NC-column system's rows (TileGeom): the doubles of a chunk of
+// row block a, the gap before chunk 2 (or every chunk), a row, and all rows
+// before block a.
+HPGL_TILE_HD constexpr int chunk_c(int nc, int a) { return (nc / 4 - (a & ~1) + 1) / 2 * 2; }
+HPGL_TILE_HD constexpr int gap_c(int nc, int a) { return chunk_c(nc, a) % 16 == 0 ? 6 : 2; }
+HPGL_TILE_HD constexpr int rbase_c(int nc, int a) {
+    int s = 0;
+    for (int q = 0; q < a; ++q) s += 4 * (4 * chunk_c(nc, q) + gap_c(nc, q));
+    return s;
+}
+
+template <int NC_, int CL_, int RL_, int PB_, int SKEW_ = 8>
+struct TileGeom {
+    static constexpr int NC = NC_, CL = CL_, RL = RL_, PB = PB_, SKEW = SKEW_;
+    static constexpr int L = CL * RL;          // lanes of a system
+    static constexpr int G = 32 / L;           // systems of a warp
+    static constexpr int NB = NC / CL;         // column blocks
+    static constexpr int H = CL / RL;          // rows of a block per lane
+    static constexpr int XN = (NC + L - 1) / L;  // rows (right-hand side) per lane
+    static_assert(NC % CL == 0 && CL % RL == 0 && 32 % L == 0, "tile shape");
+
+    // Storage of a system: rows 0..NC-1 of the upper triangle, row i (block
+    // a = i / CL) as CL chunks, chunk c holding columns c, c + CL, ... from
+    // block a (rounded down to even) on.  A lane's columns (or rows) of one
+    // row are then contiguous, 16-byte aligned pairs.  Two doubles between
+    // the chunks' halves keep the chunk starts on different 16-byte bank
+    // groups, make consecutive rows' starts (the column reads of the back
+    // substitution, one row per lane) walk through the banks, and hold
+    // RN(1 / U(i,i)) and U(i,i).
+    static_assert(CL == 4, "the chunk offsets are conflict-free for 4 chunks");
+    HPGL_TILE_HD static constexpr int cs(int a) { return chunk_c(NC, a); }
+    HPGL_TILE_HD static constexpr int chunk(int c, int a) {
+        return cs(a) % 16 == 0 ? c * (cs(a) + 2) : cs(a) % 16 == 8 ? c * cs(a) + (c & 2) : c * cs(a);
+    }
+    HPGL_TILE_HD static constexpr int pivot(int a) {
+        return cs(a) % 16 == 0 ? cs(a) : cs(a) % 16 == 8 ? 2 * cs(a) : 4 * cs(a);
+    }
+    HPGL_TILE_HD static constexpr int rstride(int a) { return CL * cs(a) + gap_c(NC, a); }
+    HPGL_TILE_HD static constexpr int rbase(int a) { return rbase_c(NC, a); }
+    // The neighbour offsets (NC 8-byte words) lie in the last rows: those of
+    // the last block, or of the last two.  The last block's covariances, the
+    // last to be gathered, are gathered before the first row of the block
+    // before it is stored.  The vectors of the outputs take the factor's place
+    // afterwards.
+    static constexpr int NBA = rbase_c(NC, NB) - rbase_c(NC, NB - 1) >= NC ? NB - 1 : NB - 2;
+    static_assert(rbase_c(NC, NB) - rbase_c(NC, NBA) >= NC, "room for the neighbour offsets");
+    static constexpr int NBAT = rbase_c(NC, NBA);
+    static constexpr int SIZE = rbase_c(NC, NB);
+    // Distance of two systems of a warp: 8-byte accesses go half a warp at a
+    // time, so where several systems share such a pass they start SKEW
+    // doubles apart in the banks.
+    static constexpr int STRIDE = SIZE + (G > 2 ? ((SKEW - SIZE) % 16 + 16) % 16 : 0);
+    static constexpr int WARP = STRIDE * (G - 1) + SIZE;
+};
+
+}  // namespace hpgl_b200
