@@ -28,9 +28,6 @@
 
 namespace hpgl_b200 {
 
-// jobs of at most this many neighbours take the exact path when mixed is asked for
-constexpr int MIXED_MIN_NEIGHBOURS = 32;
-
 #define CUDA_CHECK(expr)                                                                              \
     do {                                                                                              \
         cudaError_t e__ = (expr);                                                                     \
@@ -76,11 +73,7 @@ static int sm_count_host() {
 
 struct Counters {
     int n_untouched;
-    int n_routed;
     int err;
-    int n_attempt;         // mixed path: systems attempted in FP32
-    int n_attempt_routed;  // and of those routed
-    int abandon;           // the job was abandoned to the plain FP64 pass
     int seg_next;          // template search: the next segment (reset per launch)
     int node_next;         // clusterizer search: the next chunk of nodes (reset per launch)
     unsigned long long n_fp64;
@@ -99,7 +92,7 @@ struct Group {
 
 struct Arena {
     size_t o_values, o_codes, o_mask, o_mean, o_out_values, o_out_codes, o_out_mask, o_probs, o_pk, o_status,
-        o_variance, o_weights, o_nb, o_nbcount, o_untouched, o_routed, o_counters, o_skey, o_sidx, o_svalues,
+        o_variance, o_weights, o_nb, o_nbcount, o_untouched, o_counters, o_skey, o_sidx, o_svalues,
         o_smask, o_cross;
     size_t in_total;  // the inputs (mask, values or codes, mean cubes) come first: [0, in_total)
     size_t total;
@@ -108,8 +101,7 @@ struct Arena {
 
 struct JobState {
     hpgl_b200_job_t job;
-    int precision;   // as asked for (launch settings)
-    bool mixed;      // run the FP32 + refinement path
+    int precision;   // as asked for: selects the launch setting, the solves are FP64 for both
     long long size;
     int K;
     bool per_category;
@@ -259,12 +251,6 @@ static void prepare(JobState &S, const hpgl_b200_job_t &job, const hpgl_b200_res
     } catch (const std::invalid_argument &e) {
         throw HpglError{HPGL_E_INVALID, e.what()};
     }
-    // Up to MIXED_MIN_NEIGHBOURS neighbours the exact solve is the faster one
-    // (SK 256x256x64, 32 neighbours: 17.9 ms, an FP32 inverse with FP64
-    // refinement 22.5 ms; IK 200x200x100, 24: 9.2 and 20.7 ms), so a mixed
-    // request takes it and gets the FP64 results; its launch setting stays the
-    // mixed one's.
-    S.mixed = S.precision == HPGL_PRECISION_MIXED && S.nmax_all > MIXED_MIN_NEIGHBOURS;
     if (S.cok) {
         // cross covariance models (simple_cokriging_markI.cpp:140-181); the
         // means are mean_t (float) in the reference
@@ -329,7 +315,6 @@ static void prepare(JobState &S, const hpgl_b200_job_t &job, const hpgl_b200_res
     A.o_nb = take(n * (size_t)S.nmax_all * 4);
     A.o_nbcount = take(n * 4);
     A.o_untouched = take(n * 4);
-    A.o_routed = take(n);  // per-node routed flags
     A.o_counters = take(sizeof(Counters));
     int max_cand = 1;
     bool any_clean = false;
@@ -514,11 +499,6 @@ static DevJob make_devjob(const JobState &S, const Group &g) {
     Counters *cnt = at<Counters>(S, A.o_counters);
     J.untouched = at<int>(S, A.o_untouched);
     J.n_untouched = &cnt->n_untouched;
-    J.routed = at<uint8_t>(S, A.o_routed);
-    J.n_routed = &cnt->n_routed;
-    J.n_attempt = &cnt->n_attempt;
-    J.n_attempt_routed = &cnt->n_attempt_routed;
-    J.abandon = &cnt->abandon;
     J.seg_next = &cnt->seg_next;
     J.node_next = &cnt->node_next;
     J.n_fp64 = &cnt->n_fp64;
@@ -556,10 +536,8 @@ static void device_pass(JobState &S, cudaStream_t s, PassTiming *pt,
         Group &g = S.groups[gi];
         DevJob J = make_devjob(S, g);
         const LaunchTuning tune = tuning_get(tuning_family(g.plan.nmax), S.precision);
-        const LaunchTuning tune64 = tuning_get(tuning_family(g.plan.nmax), HPGL_PRECISION_FP64);
         if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->search0, s));
         CUDA_CHECK(cudaMemsetAsync(J.nbcount, 0, (size_t)S.size * sizeof(int), s));
-        if (S.mixed) CUDA_CHECK(cudaMemsetAsync(J.routed, 0, (size_t)S.size, s));
         launch_build_bits(J, g.dp, at<uint32_t>(S, g.o_bits), s);
         ++launches;
         if (S.cok) {
@@ -590,26 +568,16 @@ static void device_pass(JobState &S, cudaStream_t s, PassTiming *pt,
         if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top0, s));
         if (tune.schedule == SCHED_FUSED) {
             if (g.plan.nmax <= 32) launch_fused32(J, g.dp, s, tune.blocks_per_sm);
-            else launch_fused64(J, g.dp, S.mixed, s, tune.blocks_per_sm);
+            else launch_fused64(J, g.dp, s, tune.blocks_per_sm);
         } else {
-            CUDA_CHECK(cudaMemsetAsync(J.node_next, 0, sizeof(int), s));  // the mixed kernel's chunk counter
-            launch_solve(J, g.dp, S.mixed ? HPGL_PRECISION_MIXED : HPGL_PRECISION_FP64, nullptr, s, tune.blocks_per_sm);
+            CUDA_CHECK(cudaMemsetAsync(J.node_next, 0, sizeof(int), s));  // the solve's chunk counter
+            launch_solve(J, g.dp, s, tune.blocks_per_sm);
         }
         ++launches;
         if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top1, s));
-        if (S.mixed) {
-            CUDA_CHECK(cudaMemsetAsync(J.node_next, 0, sizeof(int), s));  // an abandoned job's full FP64 pass
-            launch_solve(J, g.dp, HPGL_PRECISION_FP64, J.routed, s, tune64.blocks_per_sm);
-            ++launches;
-        }
         if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->resolve1, s));
         CUDA_CHECK(cudaGetLastError());
         if (after_group) after_group(g);
-        if (S.mixed && gi + 1 < S.groups.size()) {
-            // the routed count and the job-level tally start over per group
-            CUDA_CHECK(cudaMemsetAsync(&cnt->n_routed, 0, sizeof(int), s));
-            CUDA_CHECK(cudaMemsetAsync(&cnt->n_attempt, 0, 3 * sizeof(int), s));
-        }
     }
     if (S.per_category) {
         DevJob J = make_devjob(S, S.groups[0]);
@@ -1026,13 +994,9 @@ static void sgs_run(JobState &S, hpgl_b200_result_t &res, SyncContext &C, std::c
     res.rounds = hc.rounds;
 }
 
-static const char *top_kernel_name(int nmax, bool mixed, int schedule) {
-    if (schedule == SCHED_FUSED) {
-        if (nmax <= 32) return "k_fused32";
-        return mixed ? "k_fused64<1>" : "k_fused64<0>";
-    }
-    if (nmax <= 32) return "k_solve_tile";
-    return mixed ? "k_solve_mixed64" : "k_solve_exact64";
+static const char *top_kernel_name(int nmax, int schedule) {
+    if (schedule == SCHED_FUSED) return nmax <= 32 ? "k_fused32" : "k_fused64";
+    return "k_solve_tile";
 }
 
 // The job's device pass captured once as a CUDA graph and replayed for every
@@ -1118,7 +1082,7 @@ void bench_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res, hpgl_b200_be
     bench.ms_resolve = resolve_sum / phase_runs;
     snprintf(bench.top_kernel, sizeof(bench.top_kernel), "%s",
              S.cok ? "k_cokriging"
-                   : top_kernel_name(S.nmax_all, S.mixed,
+                   : top_kernel_name(S.nmax_all,
                                      tuning_get(tuning_family(S.nmax_all), S.precision).schedule));
     bench.launches_per_iter = pt.launches;
     cudaEventDestroy(pt.search0);

@@ -314,15 +314,10 @@ void launch_search_cluster(const DevJob &J, const DevPlan &P, double *sk, int *s
     k_search_cluster<<<(unsigned)((n_warps * 32 + threads - 1) / threads), threads, 0, s>>>(J, P, sk, si, n_warps);
 }
 
-void launch_solve(const DevJob &J, const DevPlan &P, int precision, const uint8_t *routed, cudaStream_t s,
-                  int blocks_per_sm) {
+void launch_solve(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
     if (J.size <= 0) return;
-    if (P.nmax <= 32) {
-        if (!routed) launch_solve32(J, P, s, blocks_per_sm);  // nothing is ever routed
-        return;
-    }
-    if (precision == 0 || routed) launch_solve64_exact(J, P, routed, s, blocks_per_sm);
-    else launch_solve64_mixed(J, P, s, blocks_per_sm);
+    if (P.nmax <= 32) launch_solve32(J, P, s, blocks_per_sm);
+    else launch_solve64(J, P, s, blocks_per_sm);
 }
 
 // ---------------------------------------------------------------------------

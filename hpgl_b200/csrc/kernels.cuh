@@ -104,12 +104,6 @@ struct DevJob {
     // untouched nodes (ordinary kriging failures keep the caller's content)
     int *untouched;
     int *n_untouched;
-    // mixed precision routing; the job-level tally of attempts (AttemptTally)
-    uint8_t *routed;         // per node: routed to the FP64 re-solve
-    int *n_routed;
-    int *n_attempt;
-    int *n_attempt_routed;
-    int *abandon;            // set: the re-solve runs the plain FP64 pass
     int *seg_next;           // template search: the next 32-node segment to take
     int *node_next;          // clusterizer search: the next chunk of nodes to take
     // counters
@@ -159,11 +153,11 @@ void launch_build_bits(const DevJob &J, const DevPlan &P, uint32_t *bits, cudaSt
 void launch_search_template(const DevJob &J, const DevPlan &P, cudaStream_t s);
 void launch_search_cluster(const DevJob &J, const DevPlan &P, double *scratch_key, int *scratch_idx,
                            int n_warps, cudaStream_t s);
-// precision: 0 exact FP64, 1 FP32 + FP64 refinement (flags J.routed).
-// routed: optional per-node flags (the routed re-solve: the flagged nodes in
-// node order, every node once the job is abandoned); else every node.
-void launch_solve(const DevJob &J, const DevPlan &P, int precision, const uint8_t *routed, cudaStream_t s,
-                  int blocks_per_sm = 0);
+// Every node's system (the tiled FP64 solves, for either precision: an FP32
+// inverse with FP64 refinement, which mixed requests once ran, took 22.5 ms
+// where they take 17.9 at 32 neighbours and 0.82 of the one-system-a-warp
+// solve, about twice theirs, above).
+void launch_solve(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm = 0);
 void launch_ik_argmax(const DevJob &J, cudaStream_t s);
 // cokriging.cu: colocated simple cokriging of every node (after the template search)
 void launch_cokriging(const DevJob &J, const DevPlan &P, cudaStream_t s);
@@ -216,18 +210,12 @@ void launch_sis_round(const DevJob &J, const DevPlan &P0, const DevPlan *plans, 
                       int cur, cudaStream_t s);
 void launch_sis_try32(const DevJob &J, const DevPlan *plans, const SgsState &G, int cur, cudaStream_t s);
 void launch_sis_try64(const DevJob &J, const DevPlan *plans, const SgsState &G, int cur, cudaStream_t s);
-// solve32.cu: solves for max_neighbours <= 32, exact FP64 for either precision
-// (every node; the FP64 solve of the tiled kernels is faster than an FP32 one
-// with refinement was)
+// solve32.cu, solve64.cu: solves for max_neighbours <= 32 and 33..64
 void launch_solve32(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm);
-// solve64.cu: solves for 33..64 neighbours (exact FP64; FP32 inverse + FP64
-// refinement, routing to `routed`)
-void launch_solve64_exact(const DevJob &J, const DevPlan &P, const uint8_t *routed, cudaStream_t s,
-                          int blocks_per_sm);
-void launch_solve64_mixed(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm);
+void launch_solve64(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm);
 // Fused template search + solve of every node (the clusterizer search runs
-// first); precision 0 exact FP64, 1 mixed (33-64 neighbours).
+// first).
 void launch_fused32(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm);
-void launch_fused64(const DevJob &J, const DevPlan &P, int precision, cudaStream_t s, int blocks_per_sm);
+void launch_fused64(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm);
 
 }  // namespace hpgl_b200

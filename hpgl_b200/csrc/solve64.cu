@@ -1,21 +1,26 @@
-// Per-node solves for systems of 33 to 64 neighbours (one warp per system,
-// persistent over the node list; lane l owns rows and columns l and l + 32).
+// Per-node solves for systems of 33 to 64 neighbours, FP64 in the reference's
+// exact operation order (my_kriging_weights.h:26-255 over LAPACK DPOTF2 /
+// DPOTRS).
 //
-//   k_solve_exact64  FP64 in the reference's exact operation order
-//                    (my_kriging_weights.h:26-255 over LAPACK DPOTF2/DPOTRS,
-//                    the same arithmetic as the 32-neighbour kernel).  The
-//                    system and its factor live in a skewed packed upper
-//                    triangle in shared memory: every lane reads its own
-//                    columns as conflict-free 16-byte pairs while the column
-//                    of the step is broadcast, and the forward substitution
-//                    U^T y = b runs inside the factorisation (row j of U is
-//                    final at step j, which is all the dot-product form of
-//                    DTRSM needs).  The step loop is a plain runtime loop, so
-//                    the kernel stays small for the instruction caches.
+//   k_solve_tile    (tile_solve.cuh) two systems a warp, persistent over the
+//                   grid's nodes: every kriging job's solve.
+//   exact64_core    one system a warp, lane l owning rows and columns l and
+//                   l + 32: sequential simulation, the fused search + solve
+//                   kernel, and the jobs the tiled kernels do not take
+//                   (k_solve_exact64).  The system and its factor live in a
+//                   skewed packed upper triangle in shared memory: every lane
+//                   reads its own columns as conflict-free 16-byte pairs while
+//                   the column of the step is broadcast, and the forward
+//                   substitution U^T y = b runs inside the factorisation (row
+//                   j of U is final at step j, which is all the dot-product
+//                   form of DTRSM needs).  The step loop is a plain runtime
+//                   loop, so the kernel stays small for the instruction
+//                   caches.
 #include <algorithm>
 
 #include "device_common.cuh"
 #include "search_common.cuh"
+#include "tile_solve.cuh"
 
 namespace hpgl_b200 {
 
@@ -494,373 +499,41 @@ __global__ void __launch_bounds__(WARPS64_BLOCK * 32) k_sgs_try64(DevJob J, DevP
     }
 }
 
-// routed: per-node flags of the mixed pass -- the flagged nodes are solved,
-// 32 flags read at a time and taken in node order (every node once the job
-// was abandoned); null: every node.
-__global__ void __launch_bounds__(WARPS64_BLOCK * 32) k_solve_exact64(DevJob J, DevPlan P, const uint8_t *routed) {
+// Every node, for the jobs the tiled kernels do not take (tile_takes).
+__global__ void __launch_bounds__(WARPS64_BLOCK * 32) k_solve_exact64(DevJob J, DevPlan P) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     __shared__ int s_cs[N64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int k = threadIdx.x; k < N64; k += blockDim.x) s_cs[k] = col_start_c(k);
     __syncthreads();
     Exact64Smem &S = reinterpret_cast<Exact64Smem *>(dyn_smem)[warp];
-    const long long stride = (long long)gridDim.x * WARPS64_BLOCK;
     unsigned long long solved = 0;
-    long long it = (long long)blockIdx.x * WARPS64_BLOCK + warp;
-    if (routed && !*J.abandon) {
-        for (long long base = it * 32; base < J.size; base += stride * 32) {
-            const long long i = base + lane;
-            unsigned m = __ballot_sync(FULL_MASK, i < J.size && routed[i]);
-            while (m) {
-                const int k = __ffs(m) - 1;
-                m &= m - 1;
-                const NodeFetch f = fetch_node(J, P, (int)(base + k), lane);
-                solved += exact64_node(J, P, S, s_cs, f, lane);
-                __syncwarp();
-            }
-        }
-    } else {
-        // warps take up to CHUNK64 consecutive nodes at a time from a per-job
-        // counter (the next chunk taken while the current one's last node is
-        // solved), so none waits on a fixed share at the end
-        const int csize = chunk_nodes(J, CHUNK64, WARPS64_BLOCK);
-        int chunk = take_chunk64(J, lane, csize);
-        it = chunk;
-        NodeFetch cur = fetch_node(J, P, it < J.size ? (int)it : -1, lane);
-        while (it < J.size) {
-            long long nx = it + 1;
-            int nchunk = chunk;
-            if (nx == (long long)chunk + csize) {
-                nchunk = take_chunk64(J, lane, csize);
-                nx = nchunk;
-            }
-            const NodeFetch next = fetch_node(J, P, nx < J.size ? (int)nx : -1, lane);
-            solved += exact64_node(J, P, S, s_cs, cur, lane);
-            __syncwarp();
-            cur = next;
-            it = nx;
-            chunk = nchunk;
-        }
-    }
-    if (lane == 0 && solved) atomicAdd(J.n_fp64, solved);
-}
-
-// ---------------------------------------------------------------------------
-// Mixed path: FP32 Gauss-Jordan inverse + FP64 refinement.
-
-constexpr float MIXED64_PIVOT_MIN = 1e-3f;  // on the unit-diagonal scaled system
-constexpr int MIXED64_MAX_CORR = 6;
-
-struct Mixed64Smem {
-    double U[U64_SIZE];  // exact FP64 system, skewed packed upper triangle (diagonal = C(0))
-    double xv[2][N64];   // FP64 vectors broadcast for the residuals
-    float row[N64];      // pivot row of the sweep
-    float vf[2][N64];    // FP32 vectors broadcast for the inverse's products
-    int4 nb[N64];
-};
-
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-
-__device__ __forceinline__ double warp_sum64(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
-    return v;
-}
-__device__ __forceinline__ double warp_max64(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(FULL_MASK, v, o));
-    return v;
-}
-
-// (y0, y1) = rows lane and lane + 32 of M v with M's diagonal offset removed
-// (the sweep leaves every swept diagonal entry 2 above the sweep operator's
-// value; see the sweep below).
-__device__ __forceinline__ void apply64(const float2 (&m0)[32], const float2 (&m1)[32], float v0, float v1,
-                                        float *buf, int lane, float &y0, float &y1) {
-    buf[lane] = v0;
-    buf[lane + 32] = v1;
-    __syncwarp();
-    float2 a0 = f2(0.f, 0.f), a1 = f2(0.f, 0.f);
-    const float4 *b4 = reinterpret_cast<const float4 *>(buf);
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        const float4 u = b4[q];
-        a0 = __ffma2_rn(m0[2 * q], f2(u.x, u.y), a0);
-        a1 = __ffma2_rn(m1[2 * q], f2(u.x, u.y), a1);
-        a0 = __ffma2_rn(m0[2 * q + 1], f2(u.z, u.w), a0);
-        a1 = __ffma2_rn(m1[2 * q + 1], f2(u.z, u.w), a1);
-    }
-    __syncwarp();
-    y0 = (a0.x + a0.y) - 2.f * v0;
-    y1 = (a1.x + a1.y) - 2.f * v1;
-}
-
-// Rows lane and lane + 32 of r = b - A x in FP64 for one or two right-hand
-// sides; A from the packed triangle (entries of columns below n only).
-__device__ __forceinline__ void residual64(const Mixed64Smem &S, const int *cs, double a_diag, int n, int lane,
-                                           bool two, double xa0, double xa1, double xb0, double xb1,
-                                           double &ra0, double &ra1, double &rb0, double &rb1) {
-    double *xa = const_cast<double *>(S.xv[0]), *xb = const_cast<double *>(S.xv[1]);
-    xa[lane] = xa0;
-    xa[lane + 32] = xa1;
-    if (two) {
-        xb[lane] = xb0;
-        xb[lane + 32] = xb1;
-    }
-    __syncwarp();
-    const int r0 = lane, r1 = lane + 32;
-    const int cs0 = cs[r0], cs1 = cs[r1];
-    double sa0 = 0.0, sa1 = 0.0, sb0 = 0.0, sb1 = 0.0;
-    for (int k = 0; k < n; ++k) {
-        const int ck = cs[k];
-        const double a = xa[k];
-        const double b = two ? xb[k] : 0.0;
-        // A(r, k): column k at row r above the diagonal, column r at row k below
-        const double e0 = k == r0 ? a_diag : S.U[k > r0 ? ck + r0 : cs0 + k];
-        const double e1 = k == r1 ? a_diag : S.U[k > r1 ? ck + r1 : cs1 + k];
-        sa0 = fma(e0, a, sa0);
-        sa1 = fma(e1, a, sa1);
-        if (two) {
-            sb0 = fma(e0, b, sb0);
-            sb1 = fma(e1, b, sb1);
-        }
-    }
-    __syncwarp();
-    // rows from n on are padding: their residual is zero (their stale
-    // columns must not reach the inverse's products)
-    ra0 = r0 < n ? -sa0 : 0.0;
-    ra1 = r1 < n ? -sa1 : 0.0;
-    rb0 = r0 < n ? -sb0 : 0.0;
-    rb1 = r1 < n ? -sb1 : 0.0;
-}
-
-// One node of the mixed path; systems that do not qualify are appended to
-// J.routed.  skip: a system is appended at once, without the FP32 attempt.
-// Returns -1 when the node needs no system, 0 when solved here, 1 when
-// routed.
-__device__ __forceinline__ int mixed64_node(const DevJob &J, const DevPlan &P, Mixed64Smem &S, const int *cs,
-                                            const NodeFetch &cur, int lane, bool skip = false) {
-    const bool ordinary = J.kind == 0;
-    const double a_diag = __ldg(P.table + P.center);  // A(k,k) = C(0)
-    const double inv_c0 = 1.0 / P.c0;
-    const int r0 = lane, r1 = lane + 32;
-    const int cs0 = cs[r0], cs1 = cs[r1];
-    const int node = cur.node;
-    if (copy_informed64(J, cur, lane)) return -1;
-    if (skip && cur.n > 0) {
-        if (lane == 0) route(J, node);
-        __syncwarp();
-        return 1;
-    }
-    const Node64 d = load_node64(J, P, S.nb, cur, lane);
-    if (d.n <= 0) {
-        write_outputs64(J, P, node, lane, d, ST_NO_NEIGHBOURS, 0.0, 0.0, -1.0);
-        return -1;
-    }
-    const int n = d.n;
-    build_packed<false>(J, P, S.U, S.nb, cs, n, lane, nullptr);
-    // Rows lane and lane + 32 of the unit-diagonal system A / C(0),
-    // identity beyond n.
-    float2 m0[32], m1[32];
-#pragma unroll
-    for (int c = 0; c < N64; c += 2) {
-        float e[2][2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = h ? r1 : r0, csr = h ? cs1 : cs0;
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                const int cc = c + t;
-                float v;
-                if (r < n && cc < n) {
-                    const double a = cc == r ? a_diag : S.U[cc > r ? cs[cc] + r : csr + cc];
-                    v = (float)(a * inv_c0);
-                } else {
-                    v = cc == r ? 1.f : 0.f;
-                }
-                e[h][t] = v;
-            }
-        }
-        m0[c / 2] = f2(e[0][0], e[0][1]);
-        m1[c / 2] = f2(e[1][0], e[1][1]);
-    }
-    // Symmetric Gauss-Jordan sweeps over the n live rows: the matrix stays
-    // symmetric, so pivot row p (broadcast by its owner lane) is also
-    // column p and every lane reads its rows' multipliers from it.  The
-    // broadcast entry at p is set to piv - 1, which turns the same fused
-    // update into the sweep's column p (g = m_rp / piv) on every other row
-    // and leaves 2 - 1/piv in place of -1/piv on the pivot itself; swept
-    // diagonal entries are never read again, so the constant offset is
-    // removed when the inverse is applied.  After all sweeps M holds
-    // -(A/C(0))^-1 (+2 on the diagonal).
-    bool low = false;
-    for (int p = 0; p < n; ++p) {
-        const int owner = p & 31;
-        if (lane == owner) {
-            float4 *dst = reinterpret_cast<float4 *>(S.row);
-            if (p < 32) {
-#pragma unroll
-                for (int q = 0; q < 16; ++q)
-                    dst[q] = make_float4(m0[2 * q].x, m0[2 * q].y, m0[2 * q + 1].x, m0[2 * q + 1].y);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 16; ++q)
-                    dst[q] = make_float4(m1[2 * q].x, m1[2 * q].y, m1[2 * q + 1].x, m1[2 * q + 1].y);
-            }
-        }
-        __syncwarp();
-        const float piv = S.row[p];
-        if (!(piv > MIXED64_PIVOT_MIN)) {  // uniform: every lane read the same pivot
-            low = true;
-            break;
-        }
-        const float dinv = __fdividef(1.f, piv);  // approximate: the refinement absorbs it
-        const float g0 = (S.row[r0] - (r0 == p ? 1.f : 0.f)) * dinv;
-        const float g1 = (S.row[r1] - (r1 == p ? 1.f : 0.f)) * dinv;
-        __syncwarp();
-        if (lane == 0) S.row[p] = piv - 1.f;
-        __syncwarp();
-        const float2 ng0 = f2(-g0, -g0), ng1 = f2(-g1, -g1);
-        const float4 *r4 = reinterpret_cast<const float4 *>(S.row);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const float4 u = r4[q];
-            m0[2 * q] = __ffma2_rn(ng0, f2(u.x, u.y), m0[2 * q]);
-            m1[2 * q] = __ffma2_rn(ng1, f2(u.x, u.y), m1[2 * q]);
-            m0[2 * q + 1] = __ffma2_rn(ng0, f2(u.z, u.w), m0[2 * q + 1]);
-            m1[2 * q + 1] = __ffma2_rn(ng1, f2(u.z, u.w), m1[2 * q + 1]);
-        }
-        __syncwarp();
-    }
-    if (low) {
-        if (lane == 0) route(J, node);
-        __syncwarp();
-        return 1;
-    }
-    // A^-1 v = -(M v) / C(0); solutions for b (and the ones vector for OK)
-    // refined with FP64 residuals.
-    const double sc = -inv_c0;
-    const double ba0 = d.b[0], ba1 = d.b[1];
-    const double bb0 = r0 < n ? 1.0 : 0.0, bb1 = r1 < n ? 1.0 : 0.0;
-    float y0, y1;
-    apply64(m0, m1, (float)ba0, (float)ba1, S.vf[0], lane, y0, y1);
-    double xa0 = (double)y0 * sc, xa1 = (double)y1 * sc, xb0 = 0.0, xb1 = 0.0;
-    if (ordinary) {
-        apply64(m0, m1, (float)bb0, (float)bb1, S.vf[1], lane, y0, y1);
-        xb0 = (double)y0 * sc;
-        xb1 = (double)y1 * sc;
-    }
-    RefineGate gate;
-    bool converged = false;
-    for (int corr = 0; corr < MIXED64_MAX_CORR; ++corr) {
-        double ra0, ra1, rb0, rb1;
-        residual64(S, cs, a_diag, n, lane, ordinary, xa0, xa1, xb0, xb1, ra0, ra1, rb0, rb1);
-        ra0 += ba0;
-        ra1 += ba1;
-        apply64(m0, m1, (float)ra0, (float)ra1, S.vf[0], lane, y0, y1);
-        const double da0 = (double)y0 * sc, da1 = (double)y1 * sc;
-        xa0 += da0;
-        xa1 += da1;
-        double dmax = fmax(fabs(da0), fabs(da1)), xmax = fmax(fabs(xa0), fabs(xa1));
-        if (ordinary) {
-            rb0 += bb0;
-            rb1 += bb1;
-            apply64(m0, m1, (float)rb0, (float)rb1, S.vf[1], lane, y0, y1);
-            const double db0 = (double)y0 * sc, db1 = (double)y1 * sc;
-            xb0 += db0;
-            xb1 += db1;
-            dmax = fmax(dmax, fmax(fabs(db0), fabs(db1)));
-            xmax = fmax(xmax, fmax(fabs(xb0), fabs(xb1)));
-        }
-        const int decision = gate.step(warp_max64(dmax), warp_max64(xmax));
-        if (decision != 0) {
-            converged = decision > 0;
-            break;
-        }
-    }
-    if (!converged) {
-        if (lane == 0) route(J, node);
-        __syncwarp();
-        return 1;
-    }
-    if (r0 >= n) xa0 = xb0 = 0.0;
-    if (r1 >= n) xa1 = xb1 = 0.0;
-    double w0, w1;
-    if (ordinary) {
-        const double mu = (warp_sum64(xa0 + xa1) - 1.0) / warp_sum64(xb0 + xb1);
-        w0 = xa0 - mu * xb0;
-        w1 = xa1 - mu * xb1;
-    } else {
-        w0 = xa0;
-        w1 = xa1;
-    }
-    double variance = -1.0;
-    if (J.variance) {
-        // b.x* = b.x + x*.r to second order in the solution's error, with r
-        // = b - A x one more FP64 residual of the accepted solution (likewise
-        // for the ordinary-kriging sums), as residual_corrected_variance in
-        // solve32.cu
-        double qa0, qa1, qb0, qb1;
-        residual64(S, cs, a_diag, n, lane, ordinary, xa0, xa1, xb0, xb1, qa0, qa1, qb0, qb1);
-        qa0 += ba0;
-        qa1 += ba1;
-        const double bxa = warp_sum64(d.b[0] * xa0 + xa0 * qa0 + d.b[1] * xa1 + xa1 * qa1);
-        if (!ordinary) {
-            variance = P.c0 - bxa;
-        } else {
-            qb0 += bb0;
-            qb1 += bb1;
-            const double bxb = warp_sum64(d.b[0] * xb0 + xa0 * qb0 + d.b[1] * xb1 + xa1 * qb1);
-            const double oxa = warp_sum64(xa0 + xb0 * qa0 + xa1 + xb1 * qa1);
-            const double oxb = warp_sum64(xb0 + xb0 * qb0 + xb1 + xb1 * qb1);
-            const double mu = (oxa - 1.0) / oxb;
-            variance = P.c0 - (bxa - mu * bxb) - row_val(xa0 - mu * xb0, xa1 - mu * xb1, n - 1);
-        }
-    }
-    write_outputs64(J, P, node, lane, d, ST_SUCCESS, w0, w1, variance);
-    __syncwarp();
-    return 0;
-}
-
-__global__ void __launch_bounds__(32) k_solve_mixed64(DevJob J, DevPlan P) {
-    extern __shared__ __align__(16) unsigned char dyn_smem[];
-    __shared__ int s_cs[N64];
-    const int lane = threadIdx.x & 31;
-    for (int k = threadIdx.x; k < N64; k += blockDim.x) s_cs[k] = col_start_c(k);
-    __syncthreads();
-    Mixed64Smem &S = *reinterpret_cast<Mixed64Smem *>(dyn_smem);
-    // chunks of up to CHUNK64 nodes from the per-job counter, as the exact kernel;
-    // the routing guess restarts with each chunk, so its choices depend on
-    // the chunk's nodes only
-    const int csize = chunk_nodes(J, CHUNK64, 1);
+    // warps take up to CHUNK64 consecutive nodes at a time from a per-job
+    // counter (the next chunk taken while the current one's last node is
+    // solved), so none waits on a fixed share at the end
+    const int csize = chunk_nodes(J, CHUNK64, WARPS64_BLOCK);
     int chunk = take_chunk64(J, lane, csize);
     long long it = chunk;
-    NodeFetch next = fetch_node(J, P, it < J.size ? (int)it : -1, lane);
-    RouteGuess guess(ROUTE_KEEP64);
-    AttemptTally tally(ABANDON_FRACTION64);
+    NodeFetch cur = fetch_node(J, P, it < J.size ? (int)it : -1, lane);
     while (it < J.size) {
-        const NodeFetch cur = next;
-        if (it == chunk) guess = RouteGuess(ROUTE_KEEP64);
         long long nx = it + 1;
         int nchunk = chunk;
         if (nx == (long long)chunk + csize) {
             nchunk = take_chunk64(J, lane, csize);
             nx = nchunk;
         }
-        next = fetch_node(J, P, nx < J.size ? (int)nx : -1, lane);
-        const bool attempt = guess.attempt();
-        const int outcome = mixed64_node(J, P, S, s_cs, cur, lane, !attempt);
-        guess.record(attempt, outcome);
+        const NodeFetch next = fetch_node(J, P, nx < J.size ? (int)nx : -1, lane);
+        solved += exact64_node(J, P, S, s_cs, cur, lane);
         __syncwarp();
-        if (tally.step(J, attempt, outcome, lane)) break;
+        cur = next;
         it = nx;
         chunk = nchunk;
     }
+    if (lane == 0 && solved) atomicAdd(J.n_fp64, solved);
 }
 
 // Fused search + solve (one warp per block): template search of a 32-node
 // segment, then the segment's systems, as in the 32-neighbour fused kernel.
-template <int MODE>
 __global__ void __launch_bounds__(32) k_fused64(DevJob J, DevPlan P) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     __shared__ int s_cs[N64];
@@ -879,16 +552,14 @@ __global__ void __launch_bounds__(32) k_fused64(DevJob J, DevPlan P) {
         for (int b = 0; b < cnt; ++b) {
             const NodeFetch cur = next;
             next = fetch_node(J, P, b + 1 < cnt ? base + b + 1 : -1, lane);
-            if (MODE == 0) solved += exact64_node(J, P, *reinterpret_cast<Exact64Smem *>(dyn_smem), s_cs, cur, lane);
-            else mixed64_node(J, P, *reinterpret_cast<Mixed64Smem *>(dyn_smem), s_cs, cur, lane);
+            solved += exact64_node(J, P, *reinterpret_cast<Exact64Smem *>(dyn_smem), s_cs, cur, lane);
             __syncwarp();
         }
     }
-    if (MODE == 0 && lane == 0 && solved) atomicAdd(J.n_fp64, solved);
+    if (lane == 0 && solved) atomicAdd(J.n_fp64, solved);
 }
 
 constexpr size_t SMEM64_EXACT = sizeof(Exact64Smem) * WARPS64_BLOCK;
-constexpr size_t SMEM64_MIXED = sizeof(Mixed64Smem);
 
 // ---------------------------------------------------------------------------
 // Sequential indicator simulation with categories of up to 64 neighbours
@@ -986,11 +657,35 @@ __global__ void __launch_bounds__(WARPS64_BLOCK * 32) k_sis_try64(DevJob J, cons
 
 }  // namespace
 
-void launch_solve64_exact(const DevJob &J, const DevPlan &P, const uint8_t *routed, cudaStream_t s,
-                          int blocks_per_sm) {
-    const long long g = persistent_grid((const void *)k_solve_exact64, WARPS64_BLOCK * 32, SMEM64_EXACT,
-                                        blocks_per_sm, (J.size + WARPS64_BLOCK - 1) / WARPS64_BLOCK);
-    k_solve_exact64<<<(unsigned)g, WARPS64_BLOCK * 32, SMEM64_EXACT, s>>>(J, P, routed);
+// The tile of a job's systems by its largest neighbour count: 16 lanes a
+// system, 2 systems a warp (8 lanes, 4 systems: S36 31.1, 40 35.9, 48 84 ms,
+// the factors of too few systems fit an SM's shared memory), one-warp blocks,
+// as many as the factors leave room for (12 up to 40 neighbours, then 8, 7
+// and 5).  Solve of SK 256x256x64 (4.15 M systems) with the neighbour count
+// set, in ms (one system a warp, two columns a lane): 36: 28.3   40: 33.2
+// [149.6]   44: 39.8   48: 46.8 [181.7]   52: 68.0   56: 77.1 [211.3]
+// 64: 121.0 [241.7]; LVM 512x512x32 (7.5 M systems, 64) 244 [327].
+void launch_solve64(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
+    const int b = blocks_per_sm;
+    if (!tile_takes(P)) {
+        const long long g = persistent_grid((const void *)k_solve_exact64, WARPS64_BLOCK * 32, SMEM64_EXACT, b,
+                                            (J.size + WARPS64_BLOCK - 1) / WARPS64_BLOCK);
+        k_solve_exact64<<<(unsigned)g, WARPS64_BLOCK * 32, SMEM64_EXACT, s>>>(J, P);
+    } else if (P.nmax <= 36) {
+        launch_tile<TileGeom<36, 4, 4, 4>, 1, 12>(J, P, s, b);
+    } else if (P.nmax <= 40) {
+        launch_tile<TileGeom<40, 4, 4, 4>, 1, 12>(J, P, s, b);
+    } else if (P.nmax <= 44) {
+        launch_tile<TileGeom<44, 4, 4, 6>, 1, 8>(J, P, s, b);
+    } else if (P.nmax <= 48) {
+        launch_tile<TileGeom<48, 4, 4, 6>, 1, 8>(J, P, s, b);
+    } else if (P.nmax <= 52) {
+        launch_tile<TileGeom<52, 4, 4, 4>, 1, 7>(J, P, s, b);
+    } else if (P.nmax <= 56) {
+        launch_tile<TileGeom<56, 4, 4, 4>, 1, 7>(J, P, s, b);
+    } else {
+        launch_tile<TileGeom<64, 4, 4, 4>, 1, 5>(J, P, s, b);
+    }
 }
 
 void launch_sgs_try64(const DevJob &J, const DevPlan &P, const SgsState &G, int cur, cudaStream_t s) {
@@ -1004,22 +699,11 @@ void launch_sis_try64(const DevJob &J, const DevPlan *plans, const SgsState &G, 
     k_sis_try64<<<(unsigned)g, WARPS64_BLOCK * 32, smem, s>>>(J, plans, G, cur);
 }
 
-void launch_solve64_mixed(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
-    if (J.size <= 0) return;
-    const long long g = persistent_grid((const void *)k_solve_mixed64, 32, SMEM64_MIXED, blocks_per_sm, J.size);
-    k_solve_mixed64<<<(unsigned)g, 32, SMEM64_MIXED, s>>>(J, P);
-}
-
-void launch_fused64(const DevJob &J, const DevPlan &P, int precision, cudaStream_t s, int blocks_per_sm) {
+void launch_fused64(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
     const long long segs = (long long)P.nseg * J.ny * J.nz;
     if (segs <= 0) return;
-    if (precision == 0) {
-        const long long g = persistent_grid((const void *)k_fused64<0>, 32, sizeof(Exact64Smem), blocks_per_sm, segs);
-        k_fused64<0><<<(unsigned)g, 32, sizeof(Exact64Smem), s>>>(J, P);
-    } else {
-        const long long g = persistent_grid((const void *)k_fused64<1>, 32, SMEM64_MIXED, blocks_per_sm, segs);
-        k_fused64<1><<<(unsigned)g, 32, SMEM64_MIXED, s>>>(J, P);
-    }
+    const long long g = persistent_grid((const void *)k_fused64, 32, sizeof(Exact64Smem), blocks_per_sm, segs);
+    k_fused64<<<(unsigned)g, 32, sizeof(Exact64Smem), s>>>(J, P);
 }
 
 }  // namespace hpgl_b200

@@ -133,7 +133,8 @@ __device__ __forceinline__ bool tile_solve(const DevJob &J, const DevPlan &P, do
     tile_gather<T>(J, P, nb, n, r, c, 0, a[0]);
 #pragma unroll
     for (int p0 = 0; p0 < NB; ++p0) {
-        if (CL * p0 >= nw) break;
+        // no open system, or only ones that have failed
+        if (__all_sync(FULL_MASK, fail || n <= CL * p0)) break;
         const int PE = (p0 / T::PB + 1) * T::PB < NB ? (p0 / T::PB + 1) * T::PB : NB;  // the panel's end
         if (p0 > 0 && p0 % T::PB == 0) {
             // a panel's first block: the products of all finished rows

@@ -102,8 +102,11 @@ int main() {
     geometry<TileGeom<24, 4, 1, 2, 10>>();
     geometry<TileGeom<28, 4, 2, 4, 8>>();
     geometry<TileGeom<32, 4, 2, 4, 8>>();
+    geometry<TileGeom<36, 4, 4, 4>>();
     geometry<TileGeom<40, 4, 4, 4>>();
-    geometry<TileGeom<48, 4, 4, 4>>();
+    geometry<TileGeom<44, 4, 4, 6>>();
+    geometry<TileGeom<48, 4, 4, 6>>();
+    geometry<TileGeom<52, 4, 4, 4>>();
     geometry<TileGeom<56, 4, 4, 4>>();
     geometry<TileGeom<64, 4, 4, 4>>();
     packing();

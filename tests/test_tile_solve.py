@@ -86,6 +86,24 @@ def test_tile_edges_match_the_oracle(native_lib, nmax, kind):
     _check(_job(kind, nmax, (19, 13, 9), 0.12, 100 + nmax), kind)
 
 
+WIDE = [33, 36, 37, 40, 41, 44, 45, 48, 49, 52, 53, 56, 57, 63, 64]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["ok", "sk", "ik"])
+@pytest.mark.parametrize("nmax", WIDE)
+def test_wide_tile_edges_match_the_oracle(native_lib, nmax, kind):
+    _check(_job(kind, nmax, (15, 11, 7), 0.2, 200 + nmax), kind)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nmax", [40, 48, 64])
+def test_wide_singular_systems_keep_their_status(native_lib, nmax):
+    job = _job("ok", nmax, (16, 12, 8), 0.2, 6, cov=2)
+    job["params"] = [dict(job["params"][0], ranges=(90.0, 90.0, 30.0), nugget=0.0)]
+    _check(job, "ok")
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape,informed", [((1, 1, 1), 1.0), ((3, 1, 1), 0.5), ((5, 2, 1), 0.3), ((33, 1, 2), 0.05),
                                             ((17, 11, 5), 0.002), ((11, 7, 3), 0.95)])
