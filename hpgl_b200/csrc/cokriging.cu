@@ -1,6 +1,8 @@
 // Colocated simple cokriging, Markov models I and II
-// (simple_cokriging_markI.cpp:19-307), one warp per node, FP64 in the
-// reference's exact operation order.
+// (simple_cokriging_markI.cpp:19-307), FP64 in the reference's exact operation
+// order: several systems a warp on lane tiles (cok_tile.cuh), and one warp per
+// node (this file's k_cokriging) for more than 48 neighbours and for the nodes
+// whose elimination needs the search for a pivot row.
 //
 // The neighbours come from the template search (neighbour_lookup_t over the
 // untruncated primary model; the reference uses no clusterizer here).  The
@@ -13,10 +15,11 @@
 // the IEEE quotient), and eliminated from every unused row; the back
 // substitution starts each unknown from B at its own position (B[i], as the
 // reference does) and subtracts the pivot rows' terms from the last column
-// down.  The system lives row-major in shared memory; lane l owns rows l,
-// l + 32 and l + 64 (the last only for lane 0).
+// down.  In k_cokriging the system lives row-major in shared memory; lane l
+// owns rows l, l + 32 and l + 64 (the last only for lane 0).
 #include <algorithm>
 
+#include "cok_tile.cuh"
 #include "device_common.cuh"
 
 namespace hpgl_b200 {
@@ -268,7 +271,8 @@ __device__ void cok_node(const DevJob &J, const DevPlan &P, CokSmem &S, int node
     }
 }
 
-__global__ void __launch_bounds__(32) k_cokriging(DevJob J, DevPlan P) {
+// redo: the nodes the tiled kernel marked; else every node.
+__global__ void __launch_bounds__(32) k_cokriging(DevJob J, DevPlan P, bool redo) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     CokSmem S;
     {
@@ -281,17 +285,29 @@ __global__ void __launch_bounds__(32) k_cokriging(DevJob J, DevPlan P) {
     }
     const int lane = threadIdx.x & 31;
     unsigned long long solved = 0;
-    for (long long node = blockIdx.x; node < J.size; node += gridDim.x) {
-        cok_node(J, P, S, (int)node, lane, solved);
-        __syncwarp();
+    if (redo) {
+        for (long long base = (long long)blockIdx.x * 32; base < J.size; base += (long long)gridDim.x * 32) {
+            const long long i = base + lane;
+            unsigned m = __ballot_sync(FULL_MASK, i < J.size && J.status[i] == COK_REDO);
+            while (m) {
+                const int k = __ffs(m) - 1;
+                m &= m - 1;
+                cok_node(J, P, S, (int)(base + k), lane, solved);
+                __syncwarp();
+            }
+        }
+    } else {
+        for (long long node = blockIdx.x; node < J.size; node += gridDim.x) {
+            cok_node(J, P, S, (int)node, lane, solved);
+            __syncwarp();
+        }
     }
     if (lane == 0 && solved) atomicAdd(J.n_fp64, solved);
 }
 
 }  // namespace
 
-void launch_cokriging(const DevJob &J, const DevPlan &P, cudaStream_t s) {
-    if (J.size <= 0) return;
+static void launch_general(const DevJob &J, const DevPlan &P, bool redo, cudaStream_t s) {
     // the occupancy lookup is cached per kernel: ask it for the largest area,
     // and size this grid from the job's own area
     const size_t smem = cok_smem_bytes(P.nmax);
@@ -302,7 +318,45 @@ void launch_cokriging(const DevJob &J, const DevPlan &P, cudaStream_t s) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     long long g = (long long)std::max(1, per_sm) * sms;
     g = std::max<long long>(cap, std::min<long long>(g, J.size));
-    k_cokriging<<<(unsigned)g, 32, smem, s>>>(J, P);
+    if (redo) g = std::min<long long>(g, (J.size + 31) / 32);
+    k_cokriging<<<(unsigned)g, 32, smem, s>>>(J, P, redo);
+}
+
+template <typename T, int WARPS, int MINB>
+static void launch_cok_tile(const DevJob &J, const DevPlan &P, cudaStream_t s) {
+    constexpr size_t smem = sizeof(double) * T::SIZE * T::G * WARPS;
+    const long long units = (J.size + WARPS * T::G - 1) / (WARPS * T::G);
+    const long long g = persistent_grid((const void *)k_cok_tile<T, WARPS, MINB>, WARPS * 32, smem, 0, units);
+    k_cok_tile<T, WARPS, MINB><<<(unsigned)g, WARPS * 32, smem, s>>>(J, P);
+    launch_general(J, P, true, s);
+}
+
+// The tile of a job's systems by its largest neighbour count: as many lanes a
+// system as the square takes to fit the registers (4 lanes up to 12
+// neighbours, 8 up to 24, 16 up to 36, a whole warp up to 48).  Elimination of
+// 0.88 M systems (161x119x47) in ms, in brackets one system a warp with a row
+// per lane in shared memory:
+//   8: 0.44 [4.5]   12: 0.82 [6.5]   16: 1.76 [8.8]   20: 3.06 [11.2]
+//   24: 4.52 [13.7]   28: 6.65 [16.5]   36: 11.5 [26.4]   40: 17.0 [32.3]
+//   44: 19.7 [38.5]   48: 28.8 [52.6]
+// and of 4.11 M (256x256x64): 32: 38.1 [90.9].  Neighbouring tiles: 12 as 8
+// lanes 1.09, 16 as 16 lanes 2.29, 24 as 16 lanes 4.61, 32 as a whole warp
+// 47.8, 36 as a whole warp 13.6.  Above 48 the square no longer fits a warp's
+// registers.
+void launch_cokriging(const DevJob &J, const DevPlan &P, cudaStream_t s) {
+    if (J.size <= 0) return;
+    if (P.pk.m == 0 || P.nmax > 48) launch_general(J, P, false, s);
+    else if (P.nmax <= 8) launch_cok_tile<CokGeom<8, 4, 1>, 4, 4>(J, P, s);
+    else if (P.nmax <= 12) launch_cok_tile<CokGeom<12, 4, 1>, 4, 3>(J, P, s);
+    else if (P.nmax <= 16) launch_cok_tile<CokGeom<16, 4, 2>, 4, 3>(J, P, s);
+    else if (P.nmax <= 20) launch_cok_tile<CokGeom<20, 4, 2>, 4, 2>(J, P, s);
+    else if (P.nmax <= 24) launch_cok_tile<CokGeom<24, 4, 2>, 1, 7>(J, P, s);
+    else if (P.nmax <= 28) launch_cok_tile<CokGeom<28, 4, 4>, 1, 10>(J, P, s);
+    else if (P.nmax <= 32) launch_cok_tile<CokGeom<32, 4, 4>, 1, 8>(J, P, s);
+    else if (P.nmax <= 36) launch_cok_tile<CokGeom<36, 4, 4>, 1, 7>(J, P, s);
+    else if (P.nmax <= 40) launch_cok_tile<CokGeom<40, 8, 4>, 1, 10>(J, P, s);
+    else if (P.nmax <= 44) launch_cok_tile<CokGeom<44, 8, 4>, 1, 8>(J, P, s);
+    else launch_cok_tile<CokGeom<48, 8, 4>, 1, 8>(J, P, s);
 }
 
 }  // namespace hpgl_b200

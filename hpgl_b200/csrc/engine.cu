@@ -544,6 +544,7 @@ static void device_pass(JobState &S, cudaStream_t s, PassTiming *pt,
             // template search, then the cokriging systems (FP64, reference order)
             CUDA_CHECK(cudaMemsetAsync(J.seg_next, 0, sizeof(int), s));
             launch_search_template(J, g.dp, s);
+            CUDA_CHECK(cudaMemsetAsync(J.node_next, 0, sizeof(int), s));
             if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top0, s));
             launch_cokriging(J, g.dp, s);
             if (pt && gi == 0) {

@@ -1,5 +1,5 @@
-// Lane tile and shared-memory layout of a small system (tile_solve.cuh):
-// plain constants, compiled for host and device.
+// Lane tiles and shared-memory layouts of small systems (tile_solve.cuh,
+// cok_tile.cuh): plain constants, compiled for host and device.
 #pragma once
 
 #ifdef __CUDACC__
@@ -63,6 +63,32 @@ struct TileGeom {
     // doubles apart in the banks.
     static constexpr int STRIDE = SIZE + (G > 2 ? ((SKEW - SIZE) % 16 + 16) % 16 : 0);
     static constexpr int WARP = STRIDE * (G - 1) + SIZE;
+};
+
+// The square of a cokriging system (cok_tile.cuh).
+template <int NN_, int CL_, int RL_>
+struct CokGeom {
+    static constexpr int NN = NN_, CL = CL_, RL = RL_;  // NN: neighbours, even
+    static constexpr int L = CL * RL, G = 32 / L, H = CL / RL;
+    static constexpr int NBC = (NN + 2 + CL - 1) / CL;  // column blocks: NN + 1 unknowns, padding, B last
+    static constexpr int NC = CL * NBC, BCOL = NC - 1;
+    static constexpr int NBR = (NN + 1 + RL - 1) / RL;  // row blocks
+    static constexpr int NR = RL * NBR;
+    static constexpr int XN = (NN + 1 + L - 1) / L;     // unknowns per lane
+    static_assert(NN % 2 == 0 && CL % RL == 0 && 32 % L == 0 && NC > NN + 1, "tile shape");
+    // A row: CL chunks of CS doubles, chunk c the columns c, c + CL, ...; the
+    // chunk starts on different 16-byte bank groups, rows two doubles apart
+    static constexpr int even(int m) { return (m + 1) / 2 * 2; }
+    static constexpr int CS = CL == 8 && even(NBC) % 4 == 0 ? even(NBC) + 2 : even(NBC);
+    static constexpr int GAP = CL == 4 && CS % 16 == 8 ? 2 : 0;
+    static constexpr int RS = CL * CS + 2;
+    HPGL_TILE_HD static constexpr int off(int c) { return c * CS + (c & GAP); }
+    HPGL_TILE_HD static constexpr int at(int i, int k) { return i * RS + off(k % CL) + k / CL; }
+    // the pivot column, double buffered: chunk r the rows r, r + RL, ...; the
+    // neighbour offsets lie there while the system is built
+    static constexpr int CR = even(NBR) % 4 == 0 ? even(NBR) + 2 : even(NBR);
+    static constexpr int COL = NR * RS;
+    static constexpr int SIZE = COL + (2 * RL * CR > NN ? 2 * RL * CR : even(NN));
 };
 
 }  // namespace hpgl_b200

@@ -1,11 +1,12 @@
 // Compares sqrt_rcp (hpgl_b200/csrc/tile_solve.cuh: root and reciprocal root
-// together) with CUDA's IEEE operations __dsqrt_rn and __drcp_rn on the GPU:
+// together) and recip (cok_tile.cuh: a reciprocal of either sign) with CUDA's IEEE operations __dsqrt_rn and __drcp_rn on the GPU:
 // operands of kriging pivots' magnitudes, over sqrt_rcp's whole range, next to
 // squares of short numbers (roots near rounding boundaries), and next to the
 // squares of the numbers just below powers of two (divisors with a
 // significand of ones).  Prints the mismatches and exits non-zero on any.
 #include <cstdio>
 #include <cstdlib>
+#include "../../hpgl_b200/csrc/cok_tile.cuh"
 #include "../../hpgl_b200/csrc/tile_solve.cuh"
 
 __device__ unsigned long long g_bad;
@@ -39,6 +40,10 @@ __global__ void check(unsigned long long n, unsigned long long seed, int what) {
         double root, rcp;
         hpgl_b200::sqrt_rcp(a, root, rcp);
         const double r = __dsqrt_rn(a), q = __drcp_rn(r);
+        // the reciprocal of the root and of the operand, with a random sign
+        const double b = (v & 1) ? -root : (v & 2) ? -a : a;
+        double p;
+        if (!hpgl_b200::recip(b, p) || __double_as_longlong(p) != __double_as_longlong(__drcp_rn(b))) ++bad;
         if (__double_as_longlong(r) != __double_as_longlong(root) || __double_as_longlong(q) != __double_as_longlong(rcp)) ++bad;
     }
     if (bad) atomicAdd(&g_bad, bad);

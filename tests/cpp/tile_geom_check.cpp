@@ -58,6 +58,38 @@ static void geometry() {
     CHECK(T::NC <= T::SIZE);
 }
 
+template <typename T>
+static void square() {
+    std::vector<int> owner(T::SIZE, -1);
+    auto own = [&](int at, int who) {
+        CHECK(at >= 0 && at < T::SIZE);
+        if (at < 0 || at >= T::SIZE) return;
+        CHECK(owner[at] == -1);
+        owner[at] = who;
+    };
+    CHECK(T::SIZE % 2 == 0 && T::RS % 2 == 0 && T::CS % 2 == 0 && T::CR % 2 == 0 && T::COL % 2 == 0);
+    CHECK(T::NN + 1 <= T::NR && T::NR <= T::NC && T::NN + 1 < T::NC && T::BCOL == T::NC - 1);
+    CHECK(T::L * T::XN >= T::NN + 1);
+    for (int i = 0; i < T::NR; ++i)
+        for (int c = 0; c < T::CL; ++c) {
+            CHECK(T::off(c) % 2 == 0);
+            // whole pairs, as they are stored and read
+            for (int b = 0; b < T::NBC; b += 2) {
+                own(i * T::RS + T::off(c) + b, i);
+                own(i * T::RS + T::off(c) + b + 1, i);
+            }
+            for (int k = c; k < T::NC; k += T::CL) CHECK(T::at(i, k) == i * T::RS + T::off(c) + k / T::CL);
+            for (int d = 0; d < c; ++d) CHECK((T::off(c) - T::off(d)) / 2 % 8 != 0);
+        }
+    for (int q = 0; q < 2; ++q)
+        for (int r = 0; r < T::RL; ++r)
+            for (int a = 0; a < T::NBR; a += 2) {
+                own(T::COL + q * T::RL * T::CR + r * T::CR + a, 1000);
+                own(T::COL + q * T::RL * T::CR + r * T::CR + a + 1, 1000);
+            }
+    CHECK(T::COL + T::NN <= T::SIZE && T::NN + 1 <= T::COL);
+}
+
 static void packing() {
     std::mt19937 rng(1);
     auto pick = [&](int lo, int hi) { return lo + (int)(rng() % (unsigned)(hi - lo + 1)); };
@@ -109,6 +141,17 @@ int main() {
     geometry<TileGeom<52, 4, 4, 4>>();
     geometry<TileGeom<56, 4, 4, 4>>();
     geometry<TileGeom<64, 4, 4, 4>>();
+    square<CokGeom<8, 4, 1>>();
+    square<CokGeom<12, 4, 1>>();
+    square<CokGeom<16, 4, 2>>();
+    square<CokGeom<20, 4, 2>>();
+    square<CokGeom<24, 4, 2>>();
+    square<CokGeom<28, 4, 4>>();
+    square<CokGeom<32, 4, 4>>();
+    square<CokGeom<36, 4, 4>>();
+    square<CokGeom<40, 8, 4>>();
+    square<CokGeom<44, 8, 4>>();
+    square<CokGeom<48, 8, 4>>();
     packing();
     printf(bad ? "%d failures\n" : "ok\n", bad);
     return bad != 0;
