@@ -84,7 +84,7 @@ struct Counters {
 struct Group {
     int k0, k1;
     Plan plan;
-    std::vector<int4> tmpl_dev;  // device form of the template
+    RawVector<int4> tmpl_dev;  // device form of the template
     DevPlan dp;
     // arena offsets
     size_t o_tmpl, o_table, o_bstart, o_bnodes, o_bclean, o_bits;
@@ -321,8 +321,10 @@ static void prepare(JobState &S, const hpgl_b200_job_t &job, const hpgl_b200_res
     for (auto &g : S.groups) {
         const Plan &P = g.plan;
         g.tmpl_dev.resize(P.tmpl.size());
-        for (size_t i = 0; i < P.tmpl.size(); ++i)
-            g.tmpl_dev[i] = make_int4(P.px + P.tmpl[i].dx, P.tmpl[i].dy, P.tmpl[i].dz, P.tmpl[i].delta);
+        pool_for((long long)P.tmpl.size(), threads, [&](long long lo, long long hi) {
+            for (long long i = lo; i < hi; ++i)
+                g.tmpl_dev[i] = make_int4(P.px + P.tmpl[i].dx, P.tmpl[i].dy, P.tmpl[i].dz, P.tmpl[i].delta);
+        }, 32768);
         g.o_tmpl = take(g.tmpl_dev.size() * sizeof(int4));
         g.o_table = take(P.table.size() * 8);
         g.o_bstart = take(P.bucket_start.size() * 4);

@@ -44,10 +44,11 @@ static void parallel_for(long long n, int threads, F f, long long grain = 4096) 
 // evaluated as f(x, y, z).  C(v) == C(-v) bit for bit (every transformed
 // component only changes sign), so the half with z > 0 or (z == 0, y > 0) or
 // (z == y == 0, x >= 0) is evaluated and mirrored.
-template <typename F>
-static void fill_symmetric(std::vector<double> &out, int rx, int ry, int rz, int threads, F f) {
+template <typename V, typename F>
+static void fill_symmetric(V &out, int rx, int ry, int rz, int threads, F f) {
     const int xd = 2 * rx + 1, yd = 2 * ry + 1;
-    out.assign((size_t)xd * yd * (2 * rz + 1), 0.0);
+    out.clear();
+    out.resize((size_t)xd * yd * (2 * rz + 1));  // every entry is written below
     auto idx = [&](int x, int y, int z) { return ((size_t)(z + rz) * yd + (y + ry)) * xd + (x + rx); };
     // rows (z, y) of the evaluated half, z = 0..rz (y >= 0 at z = 0), a few
     // thousand covariances per thread at least
@@ -71,10 +72,57 @@ static void fill_symmetric(std::vector<double> &out, int rx, int ry, int rz, int
 // Sub-ranges above this many entries may go to another thread.
 constexpr int SORT_SPAWN_MIN = 4096;
 
+// sort_partition's result with fewer mispredicted branches (BlockQuicksort,
+// Edelkamp and Weiss, ESA 2016): the positions of the left stoppers of a block
+// of 64 at the low end and of the right stoppers of one at the high end are
+// collected without branching, and the k-th left stopper is swapped with the
+// k-th right stopper -- the pairs the scans of the Hoare partition meet one
+// after the other.  Once fewer than two blocks are left between the ends,
+// the scans themselves go on from the first unmatched stopper of each side
+// (or from the end, where a block's stoppers are used up).
+static int sort_partition_blocks(SortArr a, int lo, int hi, int pivot) {
+    constexpr int BLOCK = 64;
+    const double pk = a.key[pivot];
+    uint8_t left[BLOCK], right[BLOCK];
+    int nl = 0, nr = 0, sl = 0, sr = 0;
+    while (hi - lo > 2 * BLOCK) {
+        if (nl == 0) {
+            sl = 0;
+            for (int i = 0; i < BLOCK; ++i) {
+                left[nl] = (uint8_t)i;
+                nl += !(a.key[lo + i] > pk);
+            }
+        }
+        if (nr == 0) {
+            sr = 0;
+            for (int i = 0; i < BLOCK; ++i) {
+                right[nr] = (uint8_t)i;
+                nr += !(pk > a.key[hi - 1 - i]);
+            }
+        }
+        const int m = std::min(nl, nr);
+        for (int k = 0; k < m; ++k) a.swap(lo + left[sl + k], hi - 1 - right[sr + k]);
+        nl -= m;
+        nr -= m;
+        sl += m;
+        sr += m;
+        if (nl == 0) lo += BLOCK;
+        if (nr == 0) hi -= BLOCK;
+    }
+    if (nl) lo += left[sl];
+    if (nr) hi -= right[sr];
+    return sort_partition(a, lo, hi, pivot);
+}
+
 // The reference's std::sort permutation (introsort.h) with the independent
 // right-hand sub-ranges of large partitions sorted as pool tasks: each
 // sub-range's processing touches only its own elements, so the result is
-// the sequential algorithm's, element for element, whatever runs where.
+// the sequential algorithm's, element for element, whatever runs where.  The
+// final insertion sort only moves elements within the runs of at most 16 that
+// the partitioning leaves (no element of a later run comes before one of an
+// earlier run), so each run is inserted as soon as it is reached, while it is
+// in the cache, instead of by one pass over the whole array at the end; a
+// heap-sorted range is already in order.
 static void sort_subrange(SortArr a, int lo, int hi, int depth, TaskGroup &g) {
     while (hi - lo > 16) {
         if (depth == 0) {
@@ -84,16 +132,17 @@ static void sort_subrange(SortArr a, int lo, int hi, int depth, TaskGroup &g) {
         --depth;
         const int mid = lo + (hi - lo) / 2;
         sort_median_to_first(a, lo, lo + 1, mid, hi - 1);
-        const int cut = sort_partition(a, lo + 1, hi, lo);
+        const int cut = sort_partition_blocks(a, lo + 1, hi, lo);
         if (hi - cut > SORT_SPAWN_MIN)
             task_submit(g, [a, cut, hi, depth, &g] { sort_subrange(a, cut, hi, depth, g); });
         else
             sort_subrange(a, cut, hi, depth, g);
         hi = cut;
     }
+    sort_insertion(a, lo, hi);
 }
 
-static void parallel_reference_sort(std::vector<double> &key, std::vector<int> &idx, int threads) {
+static void parallel_reference_sort(RawVector<double> &key, RawVector<int> &idx, int threads) {
     const int n = (int)key.size();
     if (n <= 1) return;
     SortArr a{key.data(), idx.data()};
@@ -107,12 +156,6 @@ static void parallel_reference_sort(std::vector<double> &key, std::vector<int> &
     }
     task_wait(g);
     if (own) std::rethrow_exception(own);
-    if (n > 16) {
-        sort_insertion(a, 0, 16);
-        for (int i = 16; i < n; ++i) sort_linear_insert(a, i);
-    } else {
-        sort_insertion(a, 0, n);
-    }
 }
 
 // 3x3 product summed left to right, as TNT's matmult (tnt_cmat.h:472-498).
@@ -209,63 +252,81 @@ static void build_buckets(Plan &P, int nx, int ny, int nz, const KrigingParams &
     const long long nb = (long long)P.mx * P.my * P.mz;
     std::vector<int> count(nb, 0);
     std::vector<uint8_t> exceeded(nb, 0);
-    auto bucket_of = [&](long long idx) {
-        int x = (int)(idx % nx), y = (int)(idx % ((long long)nx * ny) / nx), z = (int)(idx / ((long long)nx * ny));
-        int cx = (int)(x / P.cl_r[0]), cy = (int)(y / P.cl_r[1]), cz = (int)(z / P.cl_r[2]);
-        return ((long long)cz * P.my + cy) * P.mx + cx;
-    };
-    // The informed nodes in index order (stretches of the mask scanned on all
-    // threads, eight bytes at a time).  A box takes nodes in that order until
-    // it holds `limit`, and the next one makes it overflow: it overflows
-    // exactly when it receives more than `limit` nodes.
-    std::vector<int> informed;
-    {
-        const long long chunk = std::max<long long>(1 << 16, (P.size + threads - 1) / std::max(threads, 1));
-        const long long parts = (P.size + chunk - 1) / chunk;
-        std::vector<std::vector<int>> part((size_t)parts);
-        parallel_for(parts, threads, [&](long long lo, long long hi) {
-            for (long long c = lo; c < hi; ++c) {
-                const long long a = c * chunk, e = std::min(P.size, a + chunk);
-                std::vector<int> &v = part[(size_t)c];
-                long long i = a;
-                for (; i < e && (i & 7); ++i)
-                    if (mask[i]) v.push_back((int)i);
-                for (; i + 8 <= e; i += 8) {
+    // A box takes the informed nodes in index order until it holds `limit`,
+    // and the next one makes it overflow: it overflows exactly when it
+    // receives more than `limit` nodes.  Boxes of one (y, z) strip hold the
+    // nodes of one rectangle of grid rows, so the strips are counted and
+    // filled independently, each row by row (which is index order), on all
+    // threads.
+    std::vector<int> bx(nx), ystrip(1, 0), zstrip(1, 0);  // box of x; first rows of the strips
+    for (int x = 0; x < nx; ++x) bx[x] = (int)(x / P.cl_r[0]);
+    std::vector<int> sy(1, 0), sz(1, 0);  // box of each strip
+    for (int y = 1; y < ny; ++y) {
+        const int b = (int)(y / P.cl_r[1]);
+        if (b != sy.back()) {
+            sy.push_back(b);
+            ystrip.push_back(y);
+        }
+    }
+    for (int z = 1; z < nz; ++z) {
+        const int b = (int)(z / P.cl_r[2]);
+        if (b != sz.back()) {
+            sz.push_back(b);
+            zstrip.push_back(z);
+        }
+    }
+    ystrip.push_back(ny);
+    zstrip.push_back(nz);
+    const long long strips = (long long)sy.size() * (long long)sz.size();
+    const long long grain = std::max<long long>(1, strips * 65536 / std::max<long long>(1, P.size));
+    // f(x, index, first box of the strip) over a strip's informed nodes
+    auto each_informed = [&](long long strip, auto f) {
+        const int jy = (int)(strip % (long long)sy.size()), jz = (int)(strip / (long long)sy.size());
+        const long long box = ((long long)sz[jz] * P.my + sy[jy]) * P.mx;
+        for (int z = zstrip[jz]; z < zstrip[jz + 1]; ++z)
+            for (int y = ystrip[jy]; y < ystrip[jy + 1]; ++y) {
+                const long long row = ((long long)z * ny + y) * nx;
+                const uint8_t *m = mask + row;
+                int x = 0;
+                for (; x + 8 <= nx; x += 8) {
                     uint64_t w;
-                    memcpy(&w, mask + i, 8);
+                    memcpy(&w, m + x, 8);
                     if (!w) continue;
                     for (int k = 0; k < 8; ++k)
-                        if (mask[i + k]) v.push_back((int)(i + k));
+                        if (m[x + k]) f(x + k, (int)(row + x + k), box);
                 }
-                for (; i < e; ++i)
-                    if (mask[i]) v.push_back((int)i);
+                for (; x < nx; ++x)
+                    if (m[x]) f(x, (int)(row + x), box);
             }
-        });
-        size_t total = 0;
-        for (auto &v : part) total += v.size();
-        informed.reserve(total);
-        for (auto &v : part) informed.insert(informed.end(), v.begin(), v.end());
-    }
-    P.informed = (long long)informed.size();
-    std::vector<long long> box_of(informed.size());
-    for (size_t k = 0; k < informed.size(); ++k) {
-        box_of[k] = bucket_of(informed[k]);
-        count[box_of[k]]++;
-    }
-    for (long long b = 0; b < nb; ++b)
+    };
+    parallel_for(
+        strips, threads,
+        [&](long long lo, long long hi) {
+            for (long long s = lo; s < hi; ++s) each_informed(s, [&](int x, int, long long box) { ++count[box + bx[x]]; });
+        },
+        grain);
+    P.informed = 0;
+    for (long long b = 0; b < nb; ++b) {
+        P.informed += count[b];
         if (count[b] > P.limit) {
             exceeded[b] = 1;
             count[b] = 0;
         }
+    }
     P.bucket_start.assign(nb + 1, 0);
     for (long long b = 0; b < nb; ++b) P.bucket_start[b + 1] = P.bucket_start[b] + count[b];
     P.bucket_nodes.assign(P.bucket_start[nb], 0);
-    {
+    if (P.bucket_start[nb] > 0) {
         std::vector<int> fill(P.bucket_start.begin(), P.bucket_start.end() - 1);
-        for (size_t k = 0; k < informed.size(); ++k) {
-            const long long b = box_of[k];
-            if (!exceeded[b]) P.bucket_nodes[fill[b]++] = informed[k];
-        }
+        parallel_for(
+            strips, threads,
+            [&](long long lo, long long hi) {
+                for (long long s = lo; s < hi; ++s)
+                    each_informed(s, [&](int x, int index, long long box) {
+                        if (!exceeded[box + bx[x]]) P.bucket_nodes[fill[box + bx[x]]++] = index;
+                    });
+            },
+            grain);
     }
     P.bucket_clean.assign(nb, 0);
     P.any_clean = false;
@@ -332,63 +393,82 @@ void build_plan(Plan &P, int kind, int nx, int ny, int nz, const KrigingParams &
     // pass here (the model, the precalculated table, covariance_field_t)
     // yields these same values inside the box.
     const int xd = 2 * rx + 1, yd = 2 * ry + 1;
-    std::vector<double> data;
+    RawVector<double> data;
     fill_symmetric(data, rx, ry, rz, threads, [&](int x, int y, int z) { return cov(0.0 - x, 0.0 - y, 0.0 - z); });
     lap("box");
     const double c0 = cov(0.0, 0.0, 0.0);
     const double threshold = c0 / 100;
-    // Offsets -v in z-y-x order of v, keyed by C(v) (= C(-v)); collected per
-    // z-slab in parallel and concatenated in slab order.
-    std::vector<double> keys;
-    std::vector<int> order;
-    // the template's extent: that of the offsets above the threshold,
-    // per slab while they are collected
+    // Offsets -v in z-y-x order of v, keyed by C(v) (= C(-v)): counted per
+    // z-slab in parallel (with the template's extent, that of the offsets above
+    // the threshold), then written at the slabs' places.
+    RawVector<double> keys;
+    RawVector<int> order;
     P.ext[0] = P.ext[1] = P.ext[2] = 0;
     {
         const int zd = 2 * rz + 1;
-        std::vector<std::vector<double>> kz(zd);
-        std::vector<std::vector<int>> oz(zd);
+        const long long plane = (long long)xd * yd, grain = std::max<long long>(1, 4096 / plane);
+        std::vector<size_t> start((size_t)zd + 1, 0);
         std::vector<int> ez((size_t)zd * 3, 0);
         parallel_for(
             zd, threads,
             [&](long long lo, long long hi) {
-            for (long long zi = lo; zi < hi; ++zi) {
-                const int z = (int)zi - rz;
-                int ex = 0, ey = 0;
-                for (int y = -ry; y <= ry; ++y)
-                    for (int x = -rx; x <= rx; ++x) {
-                        const double k = data[((size_t)(z + rz) * yd + (y + ry)) * xd + (x + rx)];
-                        if (k > threshold) {
-                            kz[zi].push_back(k);
-                            oz[zi].push_back((int)((((size_t)(-z + rz) * yd) + (-y + ry)) * xd + (-x + rx)));
-                            ex = std::max(ex, std::abs(x));
+                for (long long zi = lo; zi < hi; ++zi) {
+                    int ex = 0, ey = 0;
+                    size_t count = 0;
+                    for (int y = -ry; y <= ry; ++y) {
+                        const double *row = data.data() + zi * plane + (size_t)(y + ry) * xd;
+                        size_t in_row = 0;
+                        int first = xd, last = 0;
+                        for (int x = 0; x < xd; ++x)
+                            if (row[x] > threshold) {
+                                ++in_row;
+                                if (first == xd) first = x;
+                                last = x;
+                            }
+                        if (in_row) {
+                            ex = std::max(ex, std::max(std::abs(first - rx), std::abs(last - rx)));
                             ey = std::max(ey, std::abs(y));
+                            count += in_row;
                         }
                     }
-                ez[3 * zi] = ex;
-                ez[3 * zi + 1] = ey;
-                ez[3 * zi + 2] = kz[zi].empty() ? 0 : std::abs(z);
-            }
+                    start[zi + 1] = count;
+                    ez[3 * zi] = ex;
+                    ez[3 * zi + 1] = ey;
+                    ez[3 * zi + 2] = count ? std::abs((int)zi - rz) : 0;
+                }
             },
-            std::max<long long>(1, 4096 / ((long long)xd * yd)));
-        size_t total = 0;
-        for (auto &v : kz) total += v.size();
-        keys.reserve(total);
-        order.reserve(total);
+            grain);
         for (int zi = 0; zi < zd; ++zi) {
-            keys.insert(keys.end(), kz[zi].begin(), kz[zi].end());
-            order.insert(order.end(), oz[zi].begin(), oz[zi].end());
+            start[zi + 1] += start[zi];
             for (int a = 0; a < 3; ++a) P.ext[a] = std::max(P.ext[a], ez[3 * zi + a]);
         }
+        keys.resize(start[zd]);
+        order.resize(start[zd]);
+        parallel_for(
+            zd, threads,
+            [&](long long lo, long long hi) {
+                for (long long zi = lo; zi < hi; ++zi) {
+                    const int z = (int)zi - rz;
+                    size_t at = start[zi];
+                    for (int y = -ry; y <= ry && at < start[zi + 1]; ++y) {
+                        const double *row = data.data() + zi * plane + (size_t)(y + ry) * xd;
+                        for (int x = -rx; x <= rx; ++x)
+                            if (row[x + rx] > threshold) {
+                                keys[at] = row[x + rx];
+                                order[at++] = (int)((((size_t)(-z + rz) * yd) + (-y + ry)) * xd + (-x + rx));
+                            }
+                    }
+                }
+            },
+            grain);
     }
     lap("keys");
     // Every collected key is above the threshold, so the template keeps all
     // of them and the clusterizer's limit (|template| / 250) is known before
     // the sort: the buckets are built as a pool task meanwhile.
-    const int bucket_threads = std::max(1, threads / 4);
     TaskGroup bucket_task;
     task_pool_reserve(1);
-    task_submit(bucket_task, [&] { build_buckets(P, nx, ny, nz, p, mask, (long long)(keys.size() / 250), bucket_threads); });
+    task_submit(bucket_task, [&] { build_buckets(P, nx, ny, nz, p, mask, (long long)(keys.size() / 250), threads); });
     try {
         parallel_reference_sort(keys, order, threads);
     } catch (...) {

@@ -6,10 +6,30 @@
 // clusterizer buckets the reference would use.
 #pragma once
 #include <cstdint>
+#include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace hpgl_b200 {
+
+// A vector whose resize leaves new elements unset: the planning threads that
+// fill it are the first to touch its pages.
+template <typename T>
+struct RawAlloc : std::allocator<T> {
+    template <typename U>
+    struct rebind {
+        using other = RawAlloc<U>;
+    };
+    template <typename U>
+    void construct(U *) noexcept {}
+    template <typename U, typename... A>
+    void construct(U *p, A &&...a) {
+        ::new ((void *)p) U(std::forward<A>(a)...);
+    }
+};
+template <typename T>
+using RawVector = std::vector<T, RawAlloc<T>>;
 
 enum Kind { KIND_OK = 0, KIND_SK = 1, KIND_LVM = 2, KIND_IK = 3, KIND_MEDIAN_IK = 4, KIND_COK1 = 5, KIND_COK2 = 6 };
 inline bool kind_is_cokriging(int k) { return k == KIND_COK1 || k == KIND_COK2; }
@@ -55,14 +75,14 @@ struct Plan {
     int radii[3] = {0, 0, 0};
 
     // sorted search template (covariance_field.h:62-106)
-    std::vector<TemplateEntry> tmpl;
+    RawVector<TemplateEntry> tmpl;
     int ext[3] = {0, 0, 0};  // largest |offset| of the template per axis
 
     // covariance table over +-B, C(v) = table[((vz+Bz)*(2By+1) + vy+By)*(2Bx+1) + vx+Bx];
     // entries with |v| > trunc on an axis read as 0.
     int B[3] = {0, 0, 0};
     int trunc[3] = {0, 0, 0};
-    std::vector<double> table;
+    RawVector<double> table;
     double c0 = 0;  // C(0)
 
     // clusterizer (clusterizer.cpp:52-184)

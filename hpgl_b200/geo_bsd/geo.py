@@ -99,7 +99,7 @@ class IndProperty:
         self.data = numpy.require(data, "uint8", "F")
         self.mask = numpy.require(mask, "uint8", "F")
         self.indicator_count = indicator_count
-        if numpy.sum(numpy.bitwise_and(numpy.asarray(mask) > 0, numpy.asarray(data) >= indicator_count)) > 0:
+        if numpy.bitwise_and(numpy.asarray(mask) > 0, numpy.asarray(data) >= indicator_count).any():
             raise RuntimeError("Property contains some indicators outside of [0..%s] range." % (indicator_count - 1))
         assert numpy.shape(data) == numpy.shape(mask)
 
