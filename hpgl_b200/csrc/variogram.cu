@@ -8,10 +8,12 @@
 //   k_cv_offsets   one thread per window offset: tunnel test and lag range in
 //                  the reference's double arithmetic (no fused multiply-add);
 //                  the host keeps the offsets with a non-empty range;
-//   k_cv_flags / k_cv_emit   the informed cells as a compact list;
-//   k_cv_pairs     one block per (offset, slice of the cell list): each thread
-//                  accumulates its pairs' squared differences in double-double
-//                  and counts them, the block combines in a fixed order;
+//   k_cv_bits      the informed cells as padded bit rows;
+//   k_cv_flags / k_cv_emit   the words of 32 cells with any, as a compact list;
+//   k_cv_pairs     one block per (offset, slice of the word list): each thread
+//                  ands its words with the words at the offset, accumulates the
+//                  pairs' squared differences in double-double and counts them,
+//                  the block combines in a fixed order;
 //   k_cv_offset_sums, k_cv_lag_sums   fixed-order sums over slices, then over
 //                  the offsets of each lag.
 // The per-lag sums are exact to about 2^-100 relative and independent of the
@@ -196,16 +198,41 @@ struct Grid {
     int ms0, ms1, ms2;     // mask strides
 };
 
-// informed-cell flags per block of NT logical cells (x fastest)
-__global__ void k_cv_flags(Grid G, long long total, long long *block_counts) {
-    const long long i = blockIdx.x * (long long)NT + threadIdx.x;
-    bool inf = false;
-    if (i < total) {
-        const int x = (int)(i % G.nx), y = (int)((i / G.nx) % G.ny), z = (int)(i / ((long long)G.nx * G.ny));
-        inf = G.mask[(long long)x * G.ms0 + (long long)y * G.ms1 + (long long)z * G.ms2] != 0;
-    }
-    const int n = __syncthreads_count(inf);
+// The informed cells of the mask as bit rows: row (y, z) of `wpr` words, the
+// cells of x at bit `pad` words + x, zero words around them, so that a word of
+// cells displaced by any offset of the window is two words and a funnel
+// shift, zero where it leaves the mask.  One warp per word.
+__global__ void k_cv_bits(Grid G, int wx, int wpr, int pad, long long nwords, unsigned *bits) {
+    const long long i = (blockIdx.x * (long long)NT + threadIdx.x) >> 5;
+    if (i >= nwords) return;
+    const int w = (int)(i % wx), y = (int)(i / wx % G.my), z = (int)(i / ((long long)wx * G.my));
+    const int x = w * 32 + (threadIdx.x & 31);
+    const bool inf = x < G.mx && G.mask[(long long)x * G.ms0 + (long long)y * G.ms1 + (long long)z * G.ms2] != 0;
+    const unsigned b = __ballot_sync(FULL_MASK, inf);
+    if ((threadIdx.x & 31) == 0) bits[((long long)z * G.my + y) * wpr + pad + w] = b;
+}
+
+// Word i of the walked cells (the data's shape, x fastest).
+__device__ __forceinline__ unsigned walk_word(const Grid &G, const unsigned *bits, int wx, int wpr, int pad, long long i,
+                                              long long nwords, int &w, int &y, int &z) {
+    if (i >= nwords) return 0;
+    w = (int)(i % wx);
+    y = (int)(i / wx % G.ny);
+    z = (int)(i / ((long long)wx * G.ny));
+    const unsigned b = bits[((long long)z * G.my + y) * wpr + pad + w];
+    const int left = G.nx - w * 32;
+    return left < 32 ? b & ((1u << left) - 1u) : b;
+}
+
+// words with informed cells per block of NT words; the informed cells of all
+__global__ void k_cv_flags(Grid G, const unsigned *bits, int wx, int wpr, int pad, long long nwords,
+                           long long *block_counts, unsigned long long *cells) {
+    int w, y, z;
+    const unsigned b = walk_word(G, bits, wx, wpr, pad, blockIdx.x * (long long)NT + threadIdx.x, nwords, w, y, z);
+    const int n = __syncthreads_count(b != 0);
     if (threadIdx.x == 0) block_counts[blockIdx.x] = n;
+    const int c = __reduce_add_sync(FULL_MASK, __popc(b));
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(cells, (unsigned long long)c);
 }
 
 __global__ void __launch_bounds__(1024) k_cv_scan(long long *v, long long n, long long *total) {
@@ -237,27 +264,19 @@ __global__ void __launch_bounds__(1024) k_cv_scan(long long *v, long long n, lon
     if (threadIdx.x == 0) *total = tot;
 }
 
-__global__ void k_cv_emit(Grid G, long long total, const long long *block_base, int4 *cells) {
+// the words with informed cells in walk order: (word of x, y, z, cells)
+__global__ void k_cv_emit(Grid G, const unsigned *bits, int wx, int wpr, int pad, long long nwords,
+                          const long long *block_base, int4 *words) {
     __shared__ int wc[NT / 32];
-    const long long i = blockIdx.x * (long long)NT + threadIdx.x;
-    bool inf = false;
-    int x = 0, y = 0, z = 0;
-    if (i < total) {
-        x = (int)(i % G.nx);
-        y = (int)((i / G.nx) % G.ny);
-        z = (int)(i / ((long long)G.nx * G.ny));
-        inf = G.mask[(long long)x * G.ms0 + (long long)y * G.ms1 + (long long)z * G.ms2] != 0;
-    }
-    const unsigned b = __ballot_sync(FULL_MASK, inf);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) wc[w] = __popc(b);
+    int w = 0, y = 0, z = 0;
+    const unsigned cells = walk_word(G, bits, wx, wpr, pad, blockIdx.x * (long long)NT + threadIdx.x, nwords, w, y, z);
+    const unsigned b = __ballot_sync(FULL_MASK, cells != 0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) wc[warp] = __popc(b);
     __syncthreads();
     int base = 0;
-    for (int k = 0; k < w; ++k) base += wc[k];
-    if (inf) {
-        const long long pos = block_base[blockIdx.x] + base + __popc(b & ((1u << lane) - 1u));
-        cells[pos] = make_int4(x, y, z, 0);
-    }
+    for (int k = 0; k < warp; ++k) base += wc[k];
+    if (cells) words[block_base[blockIdx.x] + base + __popc(b & ((1u << lane) - 1u))] = make_int4(w, y, z, (int)cells);
 }
 
 // hash of (offset index, cell index) for percentToUse < 100
@@ -277,28 +296,46 @@ struct Offset {
     long long index;  // position in the window walk (sampling hash)
 };
 
-__global__ void __launch_bounds__(NT) k_cv_pairs(Grid G, const Offset *offs, const int4 *cells, long long ncells,
-                                                 int nchunks, long long chunk, int percent, Partial *part) {
+// One block per (offset, slice of the words): a thread ands a word of cells
+// with the word of the cells at the offset from them and visits the pairs that
+// are left.  Testing cell by cell read 16 bytes of cell and a mask byte for
+// every candidate, of which the informed share (a tenth at 10 %) are pairs:
+// 1.31 ms on 166x141x225 with 843 offsets where this takes 0.78 (6.3 and 4.0
+// at 50 % informed, 0.24 and 0.23 at 2 %); the pairs' double-double sums, a few
+// lanes of a warp at a time, bound it now.
+__global__ void __launch_bounds__(NT) k_cv_pairs(Grid G, const unsigned *bits, int wpr, int pad, const Offset *offs,
+                                                 const int4 *words, const long long *nwords, int nchunks, int percent,
+                                                 Partial *part) {
     const long long o = blockIdx.x / nchunks;
     const int ch = (int)(blockIdx.x % nchunks);
     const Offset f = offs[o];
-    const long long moff = (long long)f.x * G.ms0 + (long long)f.y * G.ms1 + (long long)f.z * G.ms2;
     const long long doff = (long long)f.x * G.ds0 + (long long)f.y * G.ds1 + (long long)f.z * G.ds2;
+    const int from = pad * 32 + f.x;
     DD acc{0.0, 0.0};
     unsigned long long n = 0;
-    const long long c0 = ch * chunk, c1 = min(ncells, c0 + chunk);
+    const long long total = *nwords, chunk = (total + nchunks - 1) / nchunks;
+    const long long c0 = ch * chunk, c1 = min(total, c0 + chunk);
     for (long long c = c0 + threadIdx.x; c < c1; c += NT) {
-        const int4 q = cells[c];
-        const int x = q.x + f.x, y = q.y + f.y, z = q.z + f.z;
-        if (x < 0 || y < 0 || z < 0 || x >= G.mx || y >= G.my || z >= G.mz) continue;
-        const long long mi = (long long)q.x * G.ms0 + (long long)q.y * G.ms1 + (long long)q.z * G.ms2;
-        if (!G.mask[mi + moff]) continue;
-        if (percent < 100 && (int)(mix2((unsigned long long)f.index, (unsigned long long)mi) % 100u) >= percent)
-            continue;
-        const long long di = (long long)q.x * G.ds0 + (long long)q.y * G.ds1 + (long long)q.z * G.ds2;
-        const double d = __dsub_rn((double)G.data[di], (double)G.data[di + doff]);
-        acc = dd_add(acc, __dmul_rn(d, d), 0.0);
-        ++n;
+        const int4 q = words[c];
+        const int y = q.y + f.y, z = q.z + f.z;
+        if ((unsigned)y >= (unsigned)G.my || (unsigned)z >= (unsigned)G.mz) continue;
+        const int xb = q.x * 32 + from;
+        const unsigned *row = bits + ((long long)z * G.my + y) * wpr + (xb >> 5);
+        unsigned m = (unsigned)q.w & __funnelshift_r(row[0], row[1], xb & 31);
+        if (!m) continue;
+        const float *d0 = G.data + (long long)q.x * 32 * G.ds0 + (long long)q.y * G.ds1 + (long long)q.z * G.ds2;
+        const long long m0 = (long long)q.x * 32 * G.ms0 + (long long)q.y * G.ms1 + (long long)q.z * G.ms2;
+        while (m) {
+            const int k = __ffs(m) - 1;
+            m &= m - 1;
+            if (percent < 100 &&
+                (int)(mix2((unsigned long long)f.index, (unsigned long long)(m0 + (long long)k * G.ms0)) % 100u) >= percent)
+                continue;
+            const float *d = d0 + (long long)k * G.ds0;
+            const double v = __dsub_rn((double)d[0], (double)d[doff]);
+            acc = dd_add(acc, __dmul_rn(v, v), 0.0);
+            ++n;
+        }
     }
     block_reduce(acc, n);
     if (threadIdx.x == 0) part[blockIdx.x] = Partial{acc.hi, acc.lo, n};
@@ -533,18 +570,40 @@ cudaStream_t cv_stream() {
     return s;
 }
 
-// device allocations freed at scope exit
+// Device memory of a call, from a pool of this file's own: freed in stream
+// order at scope exit, and up to POOL_KEEP bytes of what was freed stay with
+// the pool for the next call (a cudaMalloc and cudaFree of each buffer per
+// call took between 1 and 30 ms); more goes back to the device.
+constexpr unsigned long long POOL_KEEP = 256ull << 20;
+cudaMemPool_t cv_pool() {
+    static cudaMemPool_t pool = nullptr;
+    if (!pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        CV_CHECK(cudaGetDevice(&props.location.id));
+        cudaMemPool_t q = nullptr;
+        CV_CHECK(cudaMemPoolCreate(&q, &props));
+        unsigned long long keep = POOL_KEEP;
+        CV_CHECK(cudaMemPoolSetAttribute(q, cudaMemPoolAttrReleaseThreshold, &keep));
+        pool = q;
+    }
+    return pool;
+}
+
 struct DevMem {
+    cudaStream_t s;
     std::vector<void *> p;
+    explicit DevMem(cudaStream_t stream) : s(stream) {}
     template <typename T>
     T *alloc(size_t n) {
         void *q = nullptr;
-        CV_CHECK(cudaMalloc(&q, std::max<size_t>(n * sizeof(T), 16)));
+        CV_CHECK(cudaMallocFromPoolAsync(&q, std::max<size_t>(n * sizeof(T), 16), cv_pool(), s));
         p.push_back(q);
         return static_cast<T *>(q);
     }
     ~DevMem() {
-        for (void *q : p) cudaFree(q);
+        for (void *q : p) cudaFreeAsync(q, s);
     }
 };
 
@@ -632,7 +691,7 @@ void cv_grid(const variogram_search_template_t &t, const hard_data_t &hd, int re
     if (!hd.m_data || !hd.m_mask) throw HpglError{HPGL_E_INVALID, "data or mask is null"};
     std::lock_guard<std::mutex> lock(g_cv_mutex);
     cudaStream_t s = cv_stream();
-    DevMem M;
+    DevMem M(s);
     CallTiming timing;
     double w[6];
     window_of(t, w);
@@ -644,6 +703,13 @@ void cv_grid(const variogram_search_template_t &t, const hard_data_t &hd, int re
     const long long ncell_all = (long long)hd.m_data_shape[0] * hd.m_data_shape[1] * hd.m_data_shape[2];
     if (nwin <= 0 || ncell_all <= 0) return;
     const CvT T = cv_t(t, lags);
+    // the walked cells must lie in the mask too (the reference reads both at
+    // the same coordinates)
+    auto shapes = [&] {
+        for (int i = 0; i < 3; ++i)
+            if (hd.m_data_shape[i] > hd.m_mask_shape[i])
+                throw HpglError{HPGL_E_INVALID, "the mask is smaller than the data"};
+    };
     // offsets in the tunnel with a non-empty lag range, in the walk's order
     int2 *d_range = M.alloc<int2>((size_t)nwin);
     k_cv_offsets<<<(unsigned)((nwin + NT - 1) / NT), NT, 0, s>>>(T, i0, j0, k0, nj, nk, nwin, d_range);
@@ -651,46 +717,50 @@ void cv_grid(const variogram_search_template_t &t, const hard_data_t &hd, int re
     CV_CHECK(cudaMemcpyAsync(range.data(), d_range, (size_t)nwin * sizeof(int2), cudaMemcpyDeviceToHost, s));
     CV_CHECK(cudaStreamSynchronize(s));
     std::vector<Offset> offs;
+    bool any = false;
+    int reach = 0;
     for (long long idx = 0; idx < nwin; ++idx) {
         if (range[idx].x < 0) continue;
+        any = true;
         const int c = (int)(idx % nk), b = (int)((idx / nk) % nj), a = (int)(idx / ((long long)nk * nj));
+        // an offset as long as the mask pairs nothing
+        if (std::abs(i0 + a) >= hd.m_mask_shape[0]) continue;
         offs.push_back(Offset{i0 + a, j0 + b, k0 + c, range[idx].x, range[idx].y, idx});
+        reach = std::max(reach, std::abs(i0 + a));
     }
-    if (offs.empty()) return;
+    if (!any) return;
     // data and mask on the device
     const long long dspan = span(hd.m_data_shape, hd.m_data_strides), mspan = span(hd.m_mask_shape, hd.m_mask_strides);
     float *d_data = M.alloc<float>((size_t)dspan);
     unsigned char *d_mask = M.alloc<unsigned char>((size_t)mspan);
-    CV_CHECK(cudaMemcpyAsync(d_data, hd.m_data, (size_t)dspan * 4, cudaMemcpyHostToDevice, s));
     CV_CHECK(cudaMemcpyAsync(d_mask, hd.m_mask, (size_t)mspan, cudaMemcpyHostToDevice, s));
+    shapes();
     Grid G{d_data, d_mask, hd.m_data_shape[0], hd.m_data_shape[1], hd.m_data_shape[2], hd.m_mask_shape[0],
            hd.m_mask_shape[1], hd.m_mask_shape[2], hd.m_data_strides[0], hd.m_data_strides[1],
            hd.m_data_strides[2], hd.m_mask_strides[0], hd.m_mask_strides[1], hd.m_mask_strides[2]};
-    // the walked cells must lie in the mask too (the reference reads both at
-    // the same coordinates)
-    for (int i = 0; i < 3; ++i)
-        if (hd.m_data_shape[i] > hd.m_mask_shape[i])
-            throw HpglError{HPGL_E_INVALID, "the mask is smaller than the data"};
-    // informed cells
-    const long long nb = (ncell_all + NT - 1) / NT;
+    if (offs.empty()) return;
+    // informed cells: bit rows of the mask, and the walked words with any
+    const int wxm = (G.mx + 31) / 32, wx = (G.nx + 31) / 32, pad = (reach + 31) / 32;
+    const int wpr = wxm + 2 * pad + 1;
+    const long long mrows = (long long)G.my * G.mz, nall = mrows * wxm, nwalk = (long long)G.ny * G.nz * wx;
+    unsigned *d_bits = M.alloc<unsigned>((size_t)(mrows * wpr));
+    CV_CHECK(cudaMemsetAsync(d_bits, 0, (size_t)(mrows * wpr) * 4, s));
+    k_cv_bits<<<(unsigned)((nall * 32 + NT - 1) / NT), NT, 0, s>>>(G, wxm, wpr, pad, nall, d_bits);
+    const long long nb = (nwalk + NT - 1) / NT;
     long long *d_bc = M.alloc<long long>((size_t)nb);
-    long long *d_tot = M.alloc<long long>(1);
-    k_cv_flags<<<(unsigned)nb, NT, 0, s>>>(G, ncell_all, d_bc);
+    long long *d_tot = M.alloc<long long>(2);  // words with informed cells, informed cells
+    unsigned long long *d_cells = reinterpret_cast<unsigned long long *>(d_tot + 1);
+    CV_CHECK(cudaMemsetAsync(d_tot, 0, 16, s));
+    k_cv_flags<<<(unsigned)nb, NT, 0, s>>>(G, d_bits, wx, wpr, pad, nwalk, d_bc, d_cells);
     k_cv_scan<<<1, 1024, 0, s>>>(d_bc, nb, d_tot);
-    long long ncells = 0;
-    CV_CHECK(cudaMemcpyAsync(&ncells, d_tot, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    CV_CHECK(cudaStreamSynchronize(s));
-    if (ncells == 0) return;
-    int4 *d_cells = M.alloc<int4>((size_t)ncells);
-    k_cv_emit<<<(unsigned)nb, NT, 0, s>>>(G, ncell_all, d_bc, d_cells);
-    // (offset, slice) blocks: enough blocks to fill the GPU, slices of whole
-    // thread rows
+    int4 *d_words = M.alloc<int4>((size_t)nwalk);
+    k_cv_emit<<<(unsigned)nb, NT, 0, s>>>(G, d_bits, wx, wpr, pad, nwalk, d_bc, d_words);
+    CV_CHECK(cudaMemcpyAsync(d_data, hd.m_data, (size_t)dspan * 4, cudaMemcpyHostToDevice, s));
+    // (offset, slice) blocks: enough blocks to fill the GPU
     const long long noff = (long long)offs.size();
     const long long want_blocks = 148LL * 16;
     long long nchunks = std::max<long long>(1, (want_blocks + noff - 1) / noff);
-    nchunks = std::min<long long>(nchunks, (ncells + NT - 1) / NT);
-    const long long chunk = ((ncells + nchunks - 1) / nchunks + NT - 1) / NT * NT;
-    nchunks = (ncells + chunk - 1) / chunk;
+    nchunks = std::min<long long>(nchunks, nb);
     Offset *d_offs = M.alloc<Offset>((size_t)noff);
     CV_CHECK(cudaMemcpyAsync(d_offs, offs.data(), (size_t)noff * sizeof(Offset), cudaMemcpyHostToDevice, s));
     Partial *d_part = M.alloc<Partial>((size_t)(noff * nchunks));
@@ -700,16 +770,23 @@ void cv_grid(const variogram_search_template_t &t, const hard_data_t &hd, int re
     const long long blocks = noff * nchunks;
     if (blocks > 0x7fffffffLL) throw HpglError{HPGL_E_CAPACITY, "too many offsets for one launch"};
     CV_CHECK(cudaEventRecord(timing.e0, s));
-    k_cv_pairs<<<(unsigned)blocks, NT, 0, s>>>(G, d_offs, d_cells, ncells, (int)nchunks, chunk,
+    k_cv_pairs<<<(unsigned)blocks, NT, 0, s>>>(G, d_bits, wpr, pad, d_offs, d_words, d_tot, (int)nchunks,
                                                std::max(0, percent), d_part);
     k_cv_offset_sums<<<(unsigned)((noff * 32 + NT - 1) / NT), NT, 0, s>>>(d_part, noff, (int)nchunks, d_osum);
     k_cv_lag_sums<<<lags, NT, 0, s>>>(d_offs, d_osum, noff, d_lsum, d_ln);
     CV_CHECK(cudaEventRecord(timing.e1, s));
-    CV_CHECK(cudaMemcpyAsync(sums, d_lsum, (size_t)lags * sizeof(double), cudaMemcpyDeviceToHost, s));
-    CV_CHECK(cudaMemcpyAsync(counts, d_ln, (size_t)lags * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    unsigned long long ncells = 0;
+    std::vector<double> hs(lags);
+    std::vector<unsigned long long> hn(lags);
+    CV_CHECK(cudaMemcpyAsync(hs.data(), d_lsum, (size_t)lags * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CV_CHECK(cudaMemcpyAsync(hn.data(), d_ln, (size_t)lags * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    CV_CHECK(cudaMemcpyAsync(&ncells, d_cells, 8, cudaMemcpyDeviceToHost, s));
     CV_CHECK(cudaStreamSynchronize(s));
     CV_CHECK(cudaGetLastError());
-    timing.done(noff * ncells);
+    if (ncells == 0) return;
+    std::copy(hs.begin(), hs.end(), sums);
+    std::copy(hn.begin(), hn.end(), counts);
+    timing.done(noff * (long long)ncells);
 }
 
 void cv_points(const variogram_search_template_t &t, const cont_point_set_t &ps, int result_length, double *sums,
@@ -726,7 +803,7 @@ void cv_points(const variogram_search_template_t &t, const cont_point_set_t &ps,
     if (!ps.xs || !ps.ys || !ps.zs || !ps.values) throw HpglError{HPGL_E_INVALID, "point arrays are null"};
     std::lock_guard<std::mutex> lock(g_cv_mutex);
     cudaStream_t s = cv_stream();
-    DevMem M;
+    DevMem M(s);
     CallTiming timing;
     // lag windows (init_lag_list, variograms.cpp:140-151)
     std::vector<double> st(lags), en(lags);
@@ -791,7 +868,7 @@ void cv_stack_layers(const float_data_t *layers, const int *markers, int nlayers
     }
     std::lock_guard<std::mutex> lock(g_cv_mutex);
     cudaStream_t s = cv_stream();
-    DevMem M;
+    DevMem M(s);
     const long long lspan = span(layers[0].m_data_shape, layers[0].m_data_strides);
     std::vector<Layer> hl(nlayers);
     for (int l = 0; l < nlayers; ++l) {
