@@ -892,12 +892,34 @@ static void sgs_run(JobState &S, hpgl_b200_result_t &res, SyncContext &C, std::c
     const size_t o_ctl = take(sizeof(SgsCtl)), o_nodes = take((size_t)nsim * 4), o_xp = take((size_t)nsim * 8),
                  o_rank = take((size_t)S.size * 4), o_pend = take(bits_bytes), o_blocker = take((size_t)nsim * 4),
                  o_done = take((size_t)nsim), o_w0 = take((size_t)window * 4), o_w1 = take((size_t)window * 4),
-                 o_ok = take((size_t)window), o_try = take((size_t)window * 4);
+                 o_ok = take((size_t)window), o_try = take((size_t)window * 4),
+                 o_solve = take((size_t)window * 4);
+    // Indicator simulation: the category groups with their own search and
+    // system (two categories krige category 0 only), solved apart by the tiled
+    // kernels unless the correlogram weights scale every category's system
+    // differently, a group is not theirs, or the lists by window slot would
+    // pass 1 GiB.
+    std::vector<SisGroup> sis_groups;
+    if (indicator && !S.job.correlogram) {
+        for (auto &gr : S.groups) {
+            if (S.K == 2 && gr.k0 > 0) continue;
+            sis_groups.push_back(SisGroup{gr.dp, gr.k0, S.K == 2 ? 1 : gr.k1});
+        }
+        bool tiles = sis_groups.size() * (size_t)window * (size_t)S.nmax_all * 4 <= (size_t)1 << 30;
+        for (auto &q : sis_groups) tiles = tiles && sis_tiles(q.plan);
+        if (!tiles) sis_groups.clear();
+    }
+    const size_t lists = std::max<size_t>(1, sis_groups.size());
+    const size_t o_lists = take(lists * (size_t)window * (size_t)S.nmax_all * 4),
+                 o_counts = take(lists * (size_t)window * 4);
     std::vector<DevPlan> cat_plans;  // indicator simulation: every category's plan (its group's)
     if (indicator)
         for (auto &gr : S.groups)
             for (int k = gr.k0; k < gr.k1; ++k) cat_plans.push_back(gr.dp);
     const size_t o_plans = take(cat_plans.size() * sizeof(DevPlan));
+    std::vector<DevPlan> group_plans;
+    for (auto &q : sis_groups) group_plans.push_back(q.plan);
+    const size_t o_gplans = take(group_plans.size() * sizeof(DevPlan));
     sync_sim(C, off);
     unsigned char *scratch = C.sim;
     SgsState G;
@@ -912,7 +934,19 @@ static void sgs_run(JobState &S, hpgl_b200_result_t &res, SyncContext &C, std::c
     G.win1 = reinterpret_cast<int *>(scratch + o_w1);
     G.ok = scratch + o_ok;
     G.trylist = reinterpret_cast<int *>(scratch + o_try);
+    G.solvelist = reinterpret_cast<int *>(scratch + o_solve);
+    G.lists = reinterpret_cast<int *>(scratch + o_lists);
+    G.counts = reinterpret_cast<int *>(scratch + o_counts);
     DevPlan *d_plans = reinterpret_cast<DevPlan *>(scratch + o_plans);
+    SisGroups sis;
+    if (!sis_groups.empty()) {
+        sis.groups = sis_groups.data();
+        sis.dev = reinterpret_cast<DevPlan *>(scratch + o_gplans);
+        sis.n = (int)sis_groups.size();
+        sis.stride = S.nmax_all;
+        CUDA_CHECK(cudaMemcpyAsync(scratch + o_gplans, group_plans.data(), group_plans.size() * sizeof(DevPlan),
+                                   cudaMemcpyHostToDevice, s));
+    }
     SgsCtl hc;
     memset(&hc, 0, sizeof(hc));
     hc.window = window;
@@ -954,7 +988,7 @@ static void sgs_run(JobState &S, hpgl_b200_result_t &res, SyncContext &C, std::c
         long long committed = 0;
         for (;;) {
             for (int c = 0; c < chunk; ++c, ++round) {
-                if (indicator) launch_sis_round(J, g.dp, d_plans, S.nmax_all <= 32 ? 0 : 1, G, (int)(round & 1), s);
+                if (indicator) launch_sis_round(J, g.dp, d_plans, S.nmax_all <= 32 ? 0 : 1, sis, G, (int)(round & 1), s);
                 else launch_sgs_round(J, g.dp, G, (int)(round & 1), s);
             }
             CUDA_CHECK(cudaGetLastError());

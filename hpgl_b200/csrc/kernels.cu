@@ -342,45 +342,65 @@ __device__ __forceinline__ void sgs_bit(const DevJob &J, const DevPlan &P, int n
     bit = 1u << (px & 31);
 }
 
+// Place of this thread's entry in a list that the block appends to: one
+// update of the list's counter a block (a warp each, 8 192 updates of one
+// address a pass over the window, took longer than the pass itself).  Every
+// thread of the block calls it, `want` or not.
+__device__ __forceinline__ int block_append(bool want, int *counter, int (&warp_at)[8]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned m = __ballot_sync(FULL_MASK, want);
+    if (lane == 0) warp_at[warp] = __popc(m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int total = 0;
+        for (int w = 0; w < 8; ++w) {
+            const int c = warp_at[w];
+            warp_at[w] = total;
+            total += c;
+        }
+        const int at = total ? atomicAdd(counter, total) : 0;
+        for (int w = 0; w < 8; ++w) warp_at[w] += at;
+    }
+    __syncthreads();
+    const int at = warp_at[warp] + __popc(m & ((1u << lane) - 1u));
+    __syncthreads();
+    return at;
+}
+
 // The round's try list: the pending nodes of window buffer `cur` without a
-// blocker or whose blocker has committed (one counter update per warp); the
-// others stay pending untried.
+// blocker or whose blocker has committed; the others stay pending untried.
 __global__ void __launch_bounds__(256) k_sgs_list(SgsState G, int cur) {
+    __shared__ int warp_at[8];
     SgsCtl *ctl = G.ctl;
     const int count = ctl->count[cur];
     const int *win = cur ? G.win1 : G.win0;
-    const int lane = threadIdx.x & 31;
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < count; base += stride) {
-        const int i = base + lane;
+    const int stride = gridDim.x * 256;
+    for (int base = blockIdx.x * 256; base < count; base += stride) {
+        const int i = base + (int)threadIdx.x;
         bool tr = false;
         if (i < count) {
             const int b = G.blocker[win[i]];
             tr = b < 0 || G.done[b];
             if (!tr) G.ok[i] = 0;
         }
-        const unsigned m = __ballot_sync(FULL_MASK, tr);
-        int slot0 = 0;
-        if (lane == 0 && m) slot0 = atomicAdd(&ctl->ntry, __popc(m));
-        slot0 = __shfl_sync(FULL_MASK, slot0, 0);
-        if (tr) G.trylist[slot0 + __popc(m & ((1u << lane) - 1u))] = i;
+        const int at = block_append(tr, &ctl->ntry, warp_at);
+        if (tr) G.trylist[at] = i;
     }
 }
 
 // Commits the nodes of window buffer `cur` that the round kept (informed bit
-// set, pending bit cleared, done) and moves the others to the other buffer
-// (one counter update per warp).  The last block to finish (a ticket
-// counter, no waiting) tops the window up to its size and records the
-// admission that k_sgs_admit carries out.
+// set, pending bit cleared, done) and moves the others to the other buffer.
+// The last block to finish (a ticket counter, no waiting) tops the window up
+// to its size and records the admission that k_sgs_admit carries out.
 __global__ void __launch_bounds__(256) k_sgs_commit(DevJob J, DevPlan P, SgsState G, int cur) {
+    __shared__ int warp_at[8];
     SgsCtl *ctl = G.ctl;
     const int count = *(volatile int *)&ctl->count[cur];
     const int *win = cur ? G.win1 : G.win0;
     int *nxt = cur ? G.win0 : G.win1;
-    const int lane = threadIdx.x & 31;
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < count; base += stride) {
-        const int i = base + lane;
+    const int stride = gridDim.x * 256;
+    for (int base = blockIdx.x * 256; base < count; base += stride) {
+        const int i = base + (int)threadIdx.x;
         int rank = -1;
         bool keep = false;
         if (i < count) {
@@ -396,11 +416,8 @@ __global__ void __launch_bounds__(256) k_sgs_commit(DevJob J, DevPlan P, SgsStat
                 keep = true;
             }
         }
-        const unsigned km = __ballot_sync(FULL_MASK, keep);
-        int slot0 = 0;
-        if (lane == 0 && km) slot0 = atomicAdd(&ctl->count[cur ^ 1], __popc(km));
-        slot0 = __shfl_sync(FULL_MASK, slot0, 0);
-        if (keep) nxt[slot0 + __popc(km & ((1u << lane) - 1u))] = rank;
+        const int at = block_append(keep, &ctl->count[cur ^ 1], warp_at);
+        if (keep) nxt[at] = rank;
     }
     __shared__ bool last;
     __threadfence();
@@ -424,8 +441,10 @@ __global__ void __launch_bounds__(256) k_sgs_commit(DevJob J, DevPlan P, SgsStat
     }
     ctl->tries += ctl->ntry;
     ctl->ntry = 0;
+    ctl->nsolve = 0;
     ctl->blocks_done = 0;
     ctl->cursor = 0;
+    ctl->solve_cursor = 0;
 }
 
 // Appends the admitted path ranks to window buffer `buf` and marks them
@@ -465,10 +484,11 @@ static void sgs_list(const SgsState &G, int cur, cudaStream_t s) {
     k_sgs_list<<<(unsigned)sm_count() * 4, 256, 0, s>>>(G, cur);
 }
 
-void launch_sis_round(const DevJob &J, const DevPlan &P0, const DevPlan *plans, int family, const SgsState &G,
-                      int cur, cudaStream_t s) {
+void launch_sis_round(const DevJob &J, const DevPlan &P0, const DevPlan *plans, int family, const SisGroups &groups,
+                      const SgsState &G, int cur, cudaStream_t s) {
     sgs_list(G, cur, s);
-    if (family == 0) launch_sis_try32(J, plans, G, cur, s);
+    if (groups.n > 0) launch_sis_groups(J, groups, G, cur, s);
+    else if (family == 0) launch_sis_try32(J, plans, G, cur, s);
     else launch_sis_try64(J, plans, G, cur, s);
     sgs_commit_admit(J, P0, G, cur, s);
 }

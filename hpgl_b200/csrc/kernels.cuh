@@ -176,6 +176,8 @@ struct SgsCtl {
     unsigned blocks_done;   // commit kernel: blocks finished
     unsigned cursor;        // try kernels: next entry of the try list to hand out
     int ntry;               // entries of this round's try list
+    int nsolve;             // of those, searches that completed (solve list)
+    unsigned solve_cursor;  // next entry of the solve list to hand out
     long long next;         // next path rank to admit
     long long total;        // path length
     long long admit_base;   // window slot of the first admitted node
@@ -193,6 +195,8 @@ struct SgsState {
     int *win0, *win1;       // window buffers (path ranks)
     uint8_t *ok;            // per window slot: the node committed this round
     int *trylist;           // window slots tried this round (blocker committed or none)
+    int *solvelist;         // of those, the slots whose search completed
+    int *lists, *counts;    // per window slot (and category group): its neighbours and their number
 };
 // rank_of from the mask and the path
 void launch_sgs_ranks(const DevJob &J, const SgsState &G, long long nsim, cudaStream_t s);
@@ -205,9 +209,24 @@ void launch_sgs_try64(const DevJob &J, const DevPlan &P, const SgsState &G, int 
 void launch_sgs_admit(const DevJob &J, const DevPlan &P, const SgsState &G, int cur, cudaStream_t s);
 // sequential indicator simulation: one round over window buffer `cur` with
 // the categories' plans (device array of K); family 0 when every category
-// has at most 32 neighbours
-void launch_sis_round(const DevJob &J, const DevPlan &P0, const DevPlan *plans, int family, const SgsState &G,
-                      int cur, cudaStream_t s);
+// has at most 32 neighbours.  groups: runs of categories [k0, k1) with one
+// search and system, searched and solved apart by the tiled kernels (`n` of
+// them; their plans also on the device; the lists `stride` long), or n = 0:
+// category by category, a warp a node.
+struct SisGroup {
+    DevPlan plan;
+    int k0, k1;
+};
+struct SisGroups {
+    const SisGroup *groups = nullptr;
+    const DevPlan *dev = nullptr;
+    int n = 0, stride = 0;
+};
+// whether the tiled kernels take a plan's systems (tile_solve.cuh)
+bool sis_tiles(const DevPlan &P);
+void launch_sis_round(const DevJob &J, const DevPlan &P0, const DevPlan *plans, int family, const SisGroups &groups,
+                      const SgsState &G, int cur, cudaStream_t s);
+void launch_sis_groups(const DevJob &J, const SisGroups &groups, const SgsState &G, int cur, cudaStream_t s);
 void launch_sis_try32(const DevJob &J, const DevPlan *plans, const SgsState &G, int cur, cudaStream_t s);
 void launch_sis_try64(const DevJob &J, const DevPlan *plans, const SgsState &G, int cur, cudaStream_t s);
 // solve32.cu, solve64.cu: solves for max_neighbours <= 32 and 33..64

@@ -472,16 +472,14 @@ __device__ __forceinline__ void sgs_node32(const DevJob &J, const DevPlan &P, SM
     }
 }
 
-// One speculative round of sequential simulation (at most 32 neighbours):
-// one warp per pending node of window buffer `cur`: the template search with
+// One speculative round of sequential simulation (at most 32 neighbours) for
+// the jobs the tiled kernels do not take: one warp per pending node of window buffer `cur`: the template search with
 // conflict detection (the list in shared memory), the exact FP64 system and
 // the simulated value.
-template <int NC>
 __global__ void __launch_bounds__(WARPS32 * 32) k_sgs_try32(DevJob J, DevPlan P, SgsState G, int cur) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    using SM = SysSmemN<NC * 34>;
-    SM &S = reinterpret_cast<SM *>(dyn_smem)[warp];
+    SysSmem &S = reinterpret_cast<SysSmem *>(dyn_smem)[warp];
     const int ntry = G.ctl->ntry;
     const int *win = cur ? G.win1 : G.win0;
     // the round's tries are handed out one at a time as warps free up
@@ -493,7 +491,7 @@ __global__ void __launch_bounds__(WARPS32 * 32) k_sgs_try32(DevJob J, DevPlan P,
         const int blocker = template_node_spec(J, P, G, node, rank, lane, list, cnt);
         __syncwarp();
         if (blocker < 0) {
-            sgs_node32<NC>(J, P, S, node, list, cnt, G.xp[rank], lane);
+            sgs_node32<N32>(J, P, S, node, list, cnt, G.xp[rank], lane);
             __syncwarp();
         }
         if (lane == 0) {
@@ -547,7 +545,9 @@ __device__ __forceinline__ NodeData sis_load32(const DevJob &J, const DevPlan &P
 }
 
 // One speculative round of sequential indicator simulation (every category
-// at most 32 neighbours): one warp per pending node, the categories in
+// at most 32 neighbours) where the category groups are not solved apart: the
+// correlogram weights scale each category's system by its own means.  One warp
+// per pending node, the categories in
 // order; per category the template search with conflict detection, the
 // simple kriging system (correlogram-scaled with the mean cubes when asked)
 // and the probability m_c + sum w_i (ind_i - m_i) accumulated in double
@@ -600,15 +600,107 @@ __global__ void __launch_bounds__(WARPS32 * 32) k_sis_try32(DevJob J, const DevP
 
 }  // namespace
 
+// The searches of a simulation round on their own (the systems follow in
+// k_sgs_solve): one warp per tried node, which needs neither the registers
+// nor the shared memory of a system, so twice the warps hide the walk's
+// latency, and the finished searches' systems share warps.
+__global__ void __launch_bounds__(256) k_sgs_search(DevJob J, DevPlan P, SgsState G, int cur) {
+    const int lane = threadIdx.x & 31;
+    const int ntry = G.ctl->ntry;
+    const int *win = cur ? G.win1 : G.win0;
+    // a fixed share each: handing the tries out one at a time made the round
+    // wait for tens of thousands of updates of one counter
+    const int warps = (int)(gridDim.x * (blockDim.x >> 5));
+    for (int k = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); k < ntry; k += warps) {
+        const int slot = G.trylist[k];
+        const int rank = win[slot];
+        const int node = G.nodes[rank];
+        int cnt;
+        const int blocker = template_node_spec(J, P, G, node, rank, lane, G.lists + (long long)slot * P.nmax, cnt);
+        if (lane == 0) {
+            G.ok[slot] = blocker < 0;
+            if (blocker < 0) {
+                G.counts[slot] = cnt;
+                G.solvelist[atomicAdd(&G.ctl->nsolve, 1)] = slot;
+            } else {
+                G.blocker[rank] = blocker;
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// The searches of an indicator-simulation round: a node's category groups in
+// turn, until one meets a blocker.
+__global__ void __launch_bounds__(256) k_sis_search(DevJob J, const DevPlan *plans, int groups, int stride, SgsState G,
+                                                    int cur) {
+    const int lane = threadIdx.x & 31;
+    const int ntry = G.ctl->ntry;
+    const int *win = cur ? G.win1 : G.win0;
+    const int warps = (int)(gridDim.x * (blockDim.x >> 5));
+    for (int k = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); k < ntry; k += warps) {
+        const int slot = G.trylist[k];
+        const int rank = win[slot];
+        const int node = G.nodes[rank];
+        int blocker = -1;
+        for (int g = 0; g < groups && blocker < 0; ++g) {
+            const long long at = (long long)slot * groups + g;
+            int cnt;
+            blocker = template_node_spec(J, plans[g], G, node, rank, lane, G.lists + at * stride, cnt);
+            if (lane == 0) G.counts[at] = cnt;
+        }
+        if (lane == 0) {
+            G.ok[slot] = blocker < 0;
+            if (blocker < 0) G.solvelist[atomicAdd(&G.ctl->nsolve, 1)] = slot;
+            else G.blocker[rank] = blocker;
+        }
+        __syncwarp();
+    }
+}
+
+// Draws the codes of the round's solved nodes from their probabilities.
+__global__ void __launch_bounds__(256) k_sis_draw(DevJob J, SgsState G, int cur) {
+    const int count = G.ctl->nsolve;
+    const int *win = cur ? G.win1 : G.win0;
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < count; i += gridDim.x * 256) {
+        const int rank = win[G.solvelist[i]], node = G.nodes[rank];
+        J.sim_codes[node] = (uint8_t)sis_sample(J.probs + (long long)node * J.K, J.K, G.xp[rank]);
+        J.sim_mask[node] = 1;
+    }
+}
+
+bool sis_tiles(const DevPlan &P) { return P.nmax <= 32 && tile_takes(P); }
+
+void launch_sis_groups(const DevJob &J, const SisGroups &groups, const SgsState &G, int cur, cudaStream_t s) {
+    const long long g = persistent_grid((const void *)k_sis_search, 256, 0, 0, 1LL << 30);
+    k_sis_search<<<(unsigned)g, 256, 0, s>>>(J, groups.dev, groups.n, groups.stride, G, cur);
+    for (int i = 0; i < groups.n; ++i) {
+        const SisGroup &q = groups.groups[i];
+        const int st = groups.stride, n = groups.n, m = q.plan.nmax;
+        // the solve list is handed out once per group (the commit resets it)
+        if (i > 0) cudaMemsetAsync(&G.ctl->solve_cursor, 0, sizeof(unsigned), s);
+        if (m <= 8) launch_sis_solve<TileGeom<8, 4, 1, 2, 10>, 4, 5>(J, q.plan, G, cur, st, n, i, q.k0, q.k1, s);
+        else if (m <= 12) launch_sis_solve<TileGeom<12, 4, 1, 4, 10>, 4, 4>(J, q.plan, G, cur, st, n, i, q.k0, q.k1, s);
+        else if (m <= 16) launch_sis_solve<TileGeom<16, 4, 1, 2, 10>, 4, 3>(J, q.plan, G, cur, st, n, i, q.k0, q.k1, s);
+        else if (m <= 24) launch_sis_solve<TileGeom<24, 4, 1, 2, 10>, 4, 2>(J, q.plan, G, cur, st, n, i, q.k0, q.k1, s);
+        else launch_sis_solve<TileGeom<32, 4, 2, 4, 8>, 4, 2>(J, q.plan, G, cur, st, n, i, q.k0, q.k1, s);
+    }
+    k_sis_draw<<<(unsigned)(g < 592 ? g : 592), 256, 0, s>>>(J, G, cur);
+}
+
 void launch_sgs_try32(const DevJob &J, const DevPlan &P, const SgsState &G, int cur, cudaStream_t s) {
-    if (P.nmax <= N16) {
-        constexpr size_t smem = sizeof(SysSmem16) * WARPS32;
-        const long long g = persistent_grid((const void *)k_sgs_try32<N16>, WARPS32 * 32, smem, 0, 1LL << 30);
-        k_sgs_try32<N16><<<(unsigned)g, WARPS32 * 32, smem, s>>>(J, P, G, cur);
+    if (tile_takes(P)) {
+        const long long g = persistent_grid((const void *)k_sgs_search, 256, 0, 0, 1LL << 30);
+        k_sgs_search<<<(unsigned)g, 256, 0, s>>>(J, P, G, cur);
+        if (P.nmax <= 8) launch_sgs_solve<TileGeom<8, 4, 1, 2, 10>, 4, 5>(J, P, G, cur, s);
+        else if (P.nmax <= 12) launch_sgs_solve<TileGeom<12, 4, 1, 4, 10>, 4, 4>(J, P, G, cur, s);
+        else if (P.nmax <= 16) launch_sgs_solve<TileGeom<16, 4, 1, 2, 10>, 4, 3>(J, P, G, cur, s);
+        else if (P.nmax <= 24) launch_sgs_solve<TileGeom<24, 4, 1, 2, 10>, 4, 2>(J, P, G, cur, s);
+        else launch_sgs_solve<TileGeom<32, 4, 2, 4, 8>, 4, 2>(J, P, G, cur, s);
         return;
     }
-    const long long g = persistent_grid((const void *)k_sgs_try32<N32>, WARPS32 * 32, SMEM32, 0, 1LL << 30);
-    k_sgs_try32<N32><<<(unsigned)g, WARPS32 * 32, SMEM32, s>>>(J, P, G, cur);
+    const long long g = persistent_grid((const void *)k_sgs_try32, WARPS32 * 32, SMEM32, 0, 1LL << 30);
+    k_sgs_try32<<<(unsigned)g, WARPS32 * 32, SMEM32, s>>>(J, P, G, cur);
 }
 
 void launch_sis_try32(const DevJob &J, const DevPlan *plans, const SgsState &G, int cur, cudaStream_t s) {

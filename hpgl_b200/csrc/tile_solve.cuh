@@ -27,6 +27,7 @@
 // identity's, so they add exact zeros nowhere near the live rows.
 #pragma once
 #include "device_common.cuh"
+#include "search_common.cuh"
 #include "tile_geom.h"
 
 namespace hpgl_b200 {
@@ -472,62 +473,71 @@ __device__ __forceinline__ void tile_outputs(const DevJob &J, const DevPlan &P, 
     }
 }
 
-// Solves the warp's systems (d.node < 0: none for the group) and writes their
-// outputs; returns the number of systems solved (on every lane).
+// Solves the warp's loaded systems (d.node < 0: none for the group; nw: the
+// largest neighbour count): the group's weights and, when asked for, its kriging
+// variance.  Returns the group's status.
+template <typename T>
+__device__ __forceinline__ int tile_krige(const DevJob &J, const DevPlan &P, double *U, const TileTables<T> &B,
+                                          TileNode<T> &d, int nw, int l, bool want_variance, double (&w)[T::XN],
+                                          double &variance) {
+    const int n = d.n;
+    const bool ordinary = J.kind == 0;
+    int status = n > 0 ? ST_SUCCESS : ST_NO_NEIGHBOURS;
+#pragma unroll
+    for (int t = 0; t < T::XN; ++t) w[t] = 0.0;
+    if (nw <= 0) return status;
+    double xb[T::XN];
+#pragma unroll
+    for (int t = 0; t < T::XN; ++t) {
+        w[t] = d.b[t];
+        xb[t] = l + T::L * t < n ? 1.0 : 0.0;
+    }
+    const bool singular = ordinary ? tile_solve<T, true>(J, P, U, B, n, nw, l, w, xb)
+                                   : tile_solve<T, false>(J, P, U, B, n, nw, l, w, xb);
+    if (n > 0 && singular) status = ST_SINGULAR;
+    if (ordinary) {
+        const double ssk = tile_dsum<T>(U, 0.0, w, n, nw, l);
+        const double son = tile_dsum<T>(U, 0.0, xb, n, nw, l);
+        const double mu = __ddiv_rn(__dsub_rn(ssk, 1.0), son);
+#pragma unroll
+        for (int t = 0; t < T::XN; ++t) w[t] = __dsub_rn(w[t], __dmul_rn(mu, xb[t]));
+    }
+    if (status != ST_SUCCESS) {
+#pragma unroll
+        for (int t = 0; t < T::XN; ++t) w[t] = 0.0;
+    }
+    if (want_variance) {
+        // c0 - p_0 - p_1 - ... (my_kriging_weights.h): subtracting p is adding -p
+        double p[T::XN];
+#pragma unroll
+        for (int t = 0; t < T::XN; ++t) p[t] = -__dmul_rn(w[t], d.b[t]);
+        variance = tile_dsum<T>(U, P.c0, p, n, nw, l);
+        if (ordinary) {
+            double last = 0.0;
+            const int at = n > 0 ? n - 1 : 0;
+#pragma unroll
+            for (int t = 0; t < T::XN; ++t) {
+                const double q = __shfl_sync(FULL_MASK, w[t], at % T::L, T::L);
+                if (at / T::L == t) last = q;
+            }
+            variance = __dsub_rn(variance, last);
+        }
+    }
+    return status;
+}
+
+// The warp's systems and their outputs; returns the number of systems solved
+// (on every lane).
 template <typename T>
 __device__ __forceinline__ int tile_systems(const DevJob &J, const DevPlan &P, double *U, const TileTables<T> &B,
                                             TileNode<T> &d, int l) {
-    const int n = d.n;
-    const int nw = __reduce_max_sync(FULL_MASK, n);
-    const bool ordinary = J.kind == 0;
-    int status = n > 0 ? ST_SUCCESS : ST_NO_NEIGHBOURS;
-    double w[T::XN];
-#pragma unroll
-    for (int t = 0; t < T::XN; ++t) w[t] = 0.0;
-    double variance = -1.0;
-    if (nw > 0) {
-        tile_load<T>(J, P, U, d, l);
-        double xb[T::XN];
-#pragma unroll
-        for (int t = 0; t < T::XN; ++t) {
-            w[t] = d.b[t];
-            xb[t] = l + T::L * t < n ? 1.0 : 0.0;
-        }
-        const bool singular = ordinary ? tile_solve<T, true>(J, P, U, B, n, nw, l, w, xb)
-                                       : tile_solve<T, false>(J, P, U, B, n, nw, l, w, xb);
-        if (n > 0 && singular) status = ST_SINGULAR;
-        if (ordinary) {
-            const double ssk = tile_dsum<T>(U, 0.0, w, n, nw, l);
-            const double son = tile_dsum<T>(U, 0.0, xb, n, nw, l);
-            const double mu = __ddiv_rn(__dsub_rn(ssk, 1.0), son);
-#pragma unroll
-            for (int t = 0; t < T::XN; ++t) w[t] = __dsub_rn(w[t], __dmul_rn(mu, xb[t]));
-        }
-        if (status != ST_SUCCESS) {
-#pragma unroll
-            for (int t = 0; t < T::XN; ++t) w[t] = 0.0;
-        }
-        if (J.variance) {
-            // c0 - p_0 - p_1 - ... (my_kriging_weights.h): subtracting p is adding -p
-            double p[T::XN];
-#pragma unroll
-            for (int t = 0; t < T::XN; ++t) p[t] = -__dmul_rn(w[t], d.b[t]);
-            variance = tile_dsum<T>(U, P.c0, p, n, nw, l);
-            if (ordinary) {
-                double last = 0.0;
-                const int at = n > 0 ? n - 1 : 0;
-#pragma unroll
-                for (int t = 0; t < T::XN; ++t) {
-                    const double q = __shfl_sync(FULL_MASK, w[t], at % T::L, T::L);
-                    if (at / T::L == t) last = q;
-                }
-                variance = __dsub_rn(variance, last);
-            }
-        }
-    }
+    const int nw = __reduce_max_sync(FULL_MASK, d.n);
+    double w[T::XN], variance = -1.0;
+    if (nw > 0) tile_load<T>(J, P, U, d, l);
+    const int status = tile_krige<T>(J, P, U, B, d, nw, l, J.variance != nullptr, w, variance);
     tile_outputs<T>(J, P, U, d, nw, l, status, w, variance);
     __syncwarp();
-    return __popc(__ballot_sync(FULL_MASK, l == 0 && n > 0));
+    return __popc(__ballot_sync(FULL_MASK, l == 0 && d.n > 0));
 }
 
 // Every node of the job.  Warps take up to 32 consecutive nodes at a time from
@@ -588,10 +598,147 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_solve_tile(DevJob J, DevPl
     if (lane == 0 && solved) atomicAdd(J.n_fp64, solved);
 }
 
+// The next systems of the round's solve list, T::G at a time: the group's node,
+// its list (list `which` of the `lists` a window slot has) and path rank;
+// false once the list is used up.
+template <typename T>
+__device__ __forceinline__ bool sgs_next_systems(const SgsState &G, const int *win, int count, int stride, int lists,
+                                                 int which, int lane, TileNode<T> &d, int &rank) {
+    const int group = lane / T::L, l = lane % T::L;
+    int first = 0;
+    if (lane == 0) first = (int)atomicAdd(&G.ctl->solve_cursor, (unsigned)T::G);
+    first = __shfl_sync(FULL_MASK, first, 0);
+    if (first >= count) return false;
+    d.node = -1;
+    d.n = 0;
+    rank = 0;
+#pragma unroll
+    for (int t = 0; t < T::XN; ++t) d.cell[t] = 0;
+    if (first + group < count) {
+        const int slot = G.solvelist[first + group];
+        rank = win[slot];
+        d.node = G.nodes[rank];
+        const long long at = (long long)slot * lists + which;
+        d.n = G.counts[at];
+        const int *lst = G.lists + at * stride;
+#pragma unroll
+        for (int t = 0; t < T::XN; ++t)
+            if (l + T::L * t < d.n) d.cell[t] = lst[l + T::L * t];
+    }
+    return true;
+}
+
+// The systems of a simulation round's finished searches (G.solvelist, in any
+// order): the lists lie by window slot, and the simulated value is xp
+// sqrt(variance) + estimate, or xp where the kriging fails
+// (sequential_simulation.h:106-110, gaussian_distribution.h:49-66).
+template <typename T, int WARPS, int MINB>
+__global__ void __launch_bounds__(WARPS * 32, MINB) k_sgs_solve(DevJob J, DevPlan P, SgsState G, int cur) {
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    double *systems = reinterpret_cast<double *>(dyn_smem);
+    TileTables<T> &B = *reinterpret_cast<TileTables<T> *>(systems + tile_smem<T>(WARPS));
+    B.fill(threadIdx.x, WARPS * 32);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int group = lane / T::L, l = lane % T::L;
+    double *U = systems + warp * T::WARP + group * T::STRIDE;
+    const int count = G.ctl->nsolve;
+    const int *win = cur ? G.win1 : G.win0;
+    TileNode<T> d;
+    int rank;
+    while (sgs_next_systems<T>(G, win, count, P.nmax, 1, 0, lane, d, rank)) {
+        const bool mine = d.node >= 0;
+        const int nw = __reduce_max_sync(FULL_MASK, d.n);
+        double w[T::XN], variance = 0.0;
+        if (nw > 0) tile_load<T>(J, P, U, d, l);
+        const int status = tile_krige<T>(J, P, U, B, d, nw, l, true, w, variance);
+        float est = 0.f;
+        if (nw > 0) {
+            float term[T::XN];
+#pragma unroll
+            for (int t = 0; t < T::XN; ++t) term[t] = __double2float_rn(__dmul_rn(w[t], (double)d.dv[t]));
+            const float m0 = J.kind == 1 ? J.sk_mean_f : (J.kind == 2 && mine ? J.mean[d.node] : 0.f);
+            est = tile_fsum<T>(U, m0, term, d.n, nw, l);
+        }
+        if (mine && l == 0) {
+            const double xp = G.xp[rank];
+            const double value = status == ST_SUCCESS ? __dadd_rn(__dmul_rn(xp, __dsqrt_rn(variance)), (double)est)
+                                                      : __dadd_rn(__dmul_rn(xp, 1.0), 0.0);
+            J.sim_values[d.node] = __double2float_rn(value);
+            J.sim_mask[d.node] = 1;
+        }
+        __syncwarp();
+    }
+}
+
 // The jobs the tiled kernels take: neighbour offsets that pack into one word
 // (extents up to several hundred cells on every axis) and a sill whose pivots
 // stay in sqrt_rcp's range.  The others keep the one-system-a-warp kernels.
 inline bool tile_takes(const DevPlan &P) { return P.pk.m != 0 && P.c0 >= PIVOT_C0_MIN && P.c0 < PIVOT_C0_MAX; }
+
+// The same for indicator simulation: the system of categories [k0, k1), which
+// share a covariance model and search, solved once; per category the
+// probability m_c + sum w_i (ind_i - m_i) accumulated in double
+// (kriging_interpolation.h:228-265), the category's mean where the kriging
+// fails.  Two categories krige category 0 only and take 1 - p for the other.
+template <typename T, int WARPS, int MINB>
+__global__ void __launch_bounds__(WARPS * 32, MINB) k_sis_solve(DevJob J, DevPlan P, SgsState G, int cur, int stride,
+                                                                int lists, int which, int k0, int k1) {
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    double *systems = reinterpret_cast<double *>(dyn_smem);
+    TileTables<T> &B = *reinterpret_cast<TileTables<T> *>(systems + tile_smem<T>(WARPS));
+    B.fill(threadIdx.x, WARPS * 32);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int group = lane / T::L, l = lane % T::L;
+    double *U = systems + warp * T::WARP + group * T::STRIDE;
+    const int count = G.ctl->nsolve;
+    const int *win = cur ? G.win1 : G.win0;
+    TileNode<T> d;
+    int rank;
+    while (sgs_next_systems<T>(G, win, count, stride, lists, which, lane, d, rank)) {
+        const bool mine = d.node >= 0;
+        const int nw = __reduce_max_sync(FULL_MASK, d.n);
+        double w[T::XN], variance = 0.0;
+        if (nw > 0) tile_load<T>(J, P, U, d, l);
+        const int status = tile_krige<T>(J, P, U, B, d, nw, l, false, w, variance);
+        for (int k = k0; k < k1; ++k) {
+            const float mc = mine ? sis_mean(J, k, d.node) : 0.f;
+            double prob = (double)mc;
+            if (nw > 0) {
+                double term[T::XN];
+#pragma unroll
+                for (int t = 0; t < T::XN; ++t) {
+                    const float m = l + T::L * t < d.n ? sis_mean(J, k, d.cell[t]) : 0.f;
+                    term[t] = __dmul_rn(w[t], (double)__fsub_rn(d.code[t] == k ? 1.f : 0.f, m));
+                }
+                const double sum = tile_dsum<T>(U, (double)mc, term, d.n, nw, l);
+                if (status == ST_SUCCESS) prob = sum;
+            }
+            if (mine && l == 0) {
+                float *probs = J.probs + (long long)d.node * J.K;
+                probs[k] = __double2float_rn(prob);
+                if (J.K == 2) probs[1] = __double2float_rn(__dsub_rn(1.0, prob));
+            }
+        }
+        __syncwarp();
+    }
+}
+
+template <typename T, int WARPS, int MINB>
+static void launch_sis_solve(const DevJob &J, const DevPlan &P, const SgsState &G, int cur, int stride, int lists,
+                             int which, int k0, int k1, cudaStream_t s) {
+    constexpr size_t smem = sizeof(double) * tile_smem<T>(WARPS) + sizeof(TileTables<T>);
+    const long long g = persistent_grid((const void *)k_sis_solve<T, WARPS, MINB>, WARPS * 32, smem, 0, 1LL << 30);
+    k_sis_solve<T, WARPS, MINB><<<(unsigned)g, WARPS * 32, smem, s>>>(J, P, G, cur, stride, lists, which, k0, k1);
+}
+
+template <typename T, int WARPS, int MINB>
+static void launch_sgs_solve(const DevJob &J, const DevPlan &P, const SgsState &G, int cur, cudaStream_t s) {
+    constexpr size_t smem = sizeof(double) * tile_smem<T>(WARPS) + sizeof(TileTables<T>);
+    const long long g = persistent_grid((const void *)k_sgs_solve<T, WARPS, MINB>, WARPS * 32, smem, 0, 1LL << 30);
+    k_sgs_solve<T, WARPS, MINB><<<(unsigned)g, WARPS * 32, smem, s>>>(J, P, G, cur);
+}
 
 template <typename T, int WARPS, int MINB>
 static void launch_tile(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
