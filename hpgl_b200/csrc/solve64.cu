@@ -2,8 +2,9 @@
 // exact operation order (my_kriging_weights.h:26-255 over LAPACK DPOTF2 /
 // DPOTRS).
 //
-//   k_solve_tile    (tile_solve.cuh) two systems a warp, persistent over the
-//                   grid's nodes: every kriging job's solve.
+//   k_solve_tile    (tile_solve.cuh) two systems a warp (above 56 neighbours
+//                   one, on all its lanes), persistent over the grid's
+//                   nodes: every kriging job's solve.
 //   exact64_core    one system a warp, lane l owning rows and columns l and
 //                   l + 32: sequential simulation, the fused search + solve
 //                   kernel, and the jobs the tiled kernels do not take
@@ -657,14 +658,20 @@ __global__ void __launch_bounds__(WARPS64_BLOCK * 32) k_sis_try64(DevJob J, cons
 
 }  // namespace
 
-// The tile of a job's systems by its largest neighbour count: 16 lanes a
-// system, 2 systems a warp (8 lanes, 4 systems: S36 31.1, 40 35.9, 48 84 ms,
-// the factors of too few systems fit an SM's shared memory), one-warp blocks,
-// as many as the factors leave room for (12 up to 40 neighbours, then 8, 7
-// and 5).  Solve of SK 256x256x64 (4.15 M systems) with the neighbour count
-// set, in ms (one system a warp, two columns a lane): 36: 28.3   40: 33.2
-// [149.6]   44: 39.8   48: 46.8 [181.7]   52: 68.0   56: 77.1 [211.3]
-// 64: 121.0 [241.7]; LVM 512x512x32 (7.5 M systems, 64) 244 [327].
+// The tile of a job's systems by its largest neighbour count.  Up to 56: 16
+// lanes a system, 2 systems a warp (8 lanes, 4 systems: S36 31.1, 40 35.9, 48
+// 84 ms, the factors of too few systems fit an SM's shared memory), one-warp
+// blocks, as many as the factors leave room for (12 up to 40 neighbours, then
+// 8 and 7).  Above, two factors a warp leave room for 5 warps; 32 lanes a
+// system, 8 x 4, take half the shared memory and hold 8 warps, whose 3 200
+// more instructions a system (the pivot chain is shared by fewer) cost less
+// than the better occupancy gives: issue slots in use 48 % for 31 %.  At 56
+// and below they cost more (56: 85.2, 48: 61.0, 40: 43.8 ms).  Solve of SK
+// 256x256x64 (4.15 M systems) with the neighbour count set, in ms (one system
+// a warp, two columns a lane): 36: 28.3   40: 33.2 [149.6]   44: 39.8   48:
+// 46.8 [181.7]   52: 68.0   56: 77.1 [211.3]   64: 107.1 [241.7], 123.2 with
+// 16 lanes; LVM 512x512x32 (7.5 M systems, 64) 182.7 [327], with 16
+// lanes 244.
 void launch_solve64(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
     const int b = blocks_per_sm;
     if (!tile_takes(P)) {
@@ -684,7 +691,7 @@ void launch_solve64(const DevJob &J, const DevPlan &P, cudaStream_t s, int block
     } else if (P.nmax <= 56) {
         launch_tile<TileGeom<56, 4, 4, 4>, 1, 7>(J, P, s, b);
     } else {
-        launch_tile<TileGeom<64, 4, 4, 4>, 1, 5>(J, P, s, b);
+        launch_tile<TileGeom<64, 8, 4, 4>, 2, 4>(J, P, s, b);
     }
 }
 

@@ -10,14 +10,17 @@
 
 namespace hpgl_b200 {
 
-// Layout of an NC-column system's rows (TileGeom): the doubles of a chunk of
-// row block a, the gap before chunk 2 (or every chunk), a row, and all rows
-// before block a.
-HPGL_TILE_HD constexpr int chunk_c(int nc, int a) { return (nc / 4 - (a & ~1) + 1) / 2 * 2; }
-HPGL_TILE_HD constexpr int gap_c(int nc, int a) { return chunk_c(nc, a) % 16 == 0 ? 6 : 2; }
-HPGL_TILE_HD constexpr int rbase_c(int nc, int a) {
+// Layout of an NC-column system's rows (TileGeom), CL chunks a row: the doubles
+// of a chunk of row block a, the chunks' spread (chunk c starts at c spread +
+// its part of the gaps below), the gaps' total, and all rows before block a.
+HPGL_TILE_HD constexpr int chunk_c(int nc, int cl, int a) { return (nc / cl - (a & ~1) + 1) / 2 * 2; }
+HPGL_TILE_HD constexpr int gap_c(int nc, int cl, int a) {
+    const int cs = chunk_c(nc, cl, a);
+    return cl == 4 ? (cs % 16 == 0 ? 6 : 2) : cs % 8 == 0 ? 6 : 2;
+}
+HPGL_TILE_HD constexpr int rbase_c(int nc, int cl, int a) {
     int s = 0;
-    for (int q = 0; q < a; ++q) s += 4 * (4 * chunk_c(nc, q) + gap_c(nc, q));
+    for (int q = 0; q < a; ++q) s += cl * (cl * chunk_c(nc, cl, q) + gap_c(nc, cl, q));
     return s;
 }
 
@@ -34,30 +37,37 @@ struct TileGeom {
     // Storage of a system: rows 0..NC-1 of the upper triangle, row i (block
     // a = i / CL) as CL chunks, chunk c holding columns c, c + CL, ... from
     // block a (rounded down to even) on.  A lane's columns (or rows) of one
-    // row are then contiguous, 16-byte aligned pairs.  Two doubles between
-    // the chunks' halves keep the chunk starts on different 16-byte bank
+    // row are then contiguous, 16-byte aligned pairs.  Gaps of two doubles
+    // between chunks keep the chunk starts on different 16-byte bank
     // groups, make consecutive rows' starts (the column reads of the back
     // substitution, one row per lane) walk through the banks, and hold
     // RN(1 / U(i,i)) and U(i,i).
-    static_assert(CL == 4, "the chunk offsets are conflict-free for 4 chunks");
-    HPGL_TILE_HD static constexpr int cs(int a) { return chunk_c(NC, a); }
-    HPGL_TILE_HD static constexpr int chunk(int c, int a) {
-        return cs(a) % 16 == 0 ? c * (cs(a) + 2) : cs(a) % 16 == 8 ? c * cs(a) + (c & 2) : c * cs(a);
+    static_assert(CL == 4 || (CL == 8 && NB < 16), "the chunk offsets are conflict-free for 4 and 8 chunks");
+    HPGL_TILE_HD static constexpr int cs(int a) { return chunk_c(NC, CL, a); }
+    // chunk c starts at c spread(a) + (c & mask(a)) / (shift(a) ? 2 : 1)
+    HPGL_TILE_HD static constexpr int spread(int a) { return CL == 4 && cs(a) % 16 == 0 ? cs(a) + 2 : cs(a); }
+    HPGL_TILE_HD static constexpr int mask(int a) {
+        return CL == 4 ? (cs(a) % 16 == 8 ? 2 : 0) : cs(a) % 8 == 0 ? 6 : cs(a) % 8 == 4 ? 4 : 0;
     }
+    HPGL_TILE_HD static constexpr int shift(int a) { return CL == 8 && cs(a) % 8 == 4 ? 1 : 0; }
+    HPGL_TILE_HD static constexpr int chunk(int c, int a) { return c * spread(a) + ((c & mask(a)) >> shift(a)); }
     HPGL_TILE_HD static constexpr int pivot(int a) {
-        return cs(a) % 16 == 0 ? cs(a) : cs(a) % 16 == 8 ? 2 * cs(a) : 4 * cs(a);
+        return CL == 4 && cs(a) % 16 == 0 ? cs(a)
+               : mask(a) == 0             ? CL * cs(a)
+               : mask(a) == 4             ? 4 * cs(a)
+                                          : 2 * cs(a);
     }
-    HPGL_TILE_HD static constexpr int rstride(int a) { return CL * cs(a) + gap_c(NC, a); }
-    HPGL_TILE_HD static constexpr int rbase(int a) { return rbase_c(NC, a); }
+    HPGL_TILE_HD static constexpr int rstride(int a) { return CL * cs(a) + gap_c(NC, CL, a); }
+    HPGL_TILE_HD static constexpr int rbase(int a) { return rbase_c(NC, CL, a); }
     // The neighbour offsets (NC 8-byte words) lie in the last rows: those of
     // the last block, or of the last two.  The last block's covariances, the
     // last to be gathered, are gathered before the first row of the block
     // before it is stored.  The vectors of the outputs take the factor's place
     // afterwards.
-    static constexpr int NBA = rbase_c(NC, NB) - rbase_c(NC, NB - 1) >= NC ? NB - 1 : NB - 2;
-    static_assert(rbase_c(NC, NB) - rbase_c(NC, NBA) >= NC, "room for the neighbour offsets");
-    static constexpr int NBAT = rbase_c(NC, NBA);
-    static constexpr int SIZE = rbase_c(NC, NB);
+    static constexpr int NBA = rbase_c(NC, CL, NB) - rbase_c(NC, CL, NB - 1) >= NC ? NB - 1 : NB - 2;
+    static_assert(rbase_c(NC, CL, NB) - rbase_c(NC, CL, NBA) >= NC, "room for the neighbour offsets");
+    static constexpr int NBAT = rbase_c(NC, CL, NBA);
+    static constexpr int SIZE = rbase_c(NC, CL, NB);
     // Distance of two systems of a warp: 8-byte accesses go half a warp at a
     // time, so where several systems share such a pass they start SKEW
     // doubles apart in the banks.

@@ -33,7 +33,7 @@
 namespace hpgl_b200 {
 
 // Per-block table of row i: U(i, k) = U[x + chunk(k % CL) + k / CL], with the
-// chunk's offset (k % CL) y + (k % CL & z).
+// chunk's offset (k % CL) y + ((k % CL & z) >> w).
 template <typename T>
 struct alignas(16) TileTables {
     short4 row[T::NC];
@@ -41,8 +41,12 @@ struct alignas(16) TileTables {
         for (int i = thread; i < T::NC; i += threads) {
             const int a = i / T::CL;
             row[i] = make_short4((short)(T::rbase(a) + (i % T::CL) * T::rstride(a) - (a & ~1)),
-                                 (short)T::chunk(1, a), (short)(T::cs(a) % 16 == 8 ? 2 : 0), 0);
+                                 (short)T::spread(a), (short)T::mask(a), (short)T::shift(a));
         }
+    }
+    // chunk c of row q
+    static __device__ __forceinline__ int chunk(const short4 &q, int c) {
+        return c * q.y + (T::CL == 4 ? c & q.z : (c & q.z) >> q.w);
     }
 };
 
@@ -142,7 +146,7 @@ __device__ __forceinline__ bool tile_solve(const DevJob &J, const DevPlan &P, do
 #pragma unroll 2
             for (int j = 0; j < CL * p0; ++j) {
                 const short4 q = B.row[j];
-                const double *colp = U + q.x + c * q.y + (c & q.z);
+                const double *colp = U + q.x + B.chunk(q, c);
                 double cu[NB + 1];
 #pragma unroll
                 for (int b = p0; b < NB; b += 2) {
@@ -152,7 +156,7 @@ __device__ __forceinline__ bool tile_solve(const DevJob &J, const DevPlan &P, do
                 }
 #pragma unroll
                 for (int h = 0; h < H; ++h) {
-                    const double *rowp = U + q.x + (r + RL * h) * q.y + ((r + RL * h) & q.z);
+                    const double *rowp = U + q.x + B.chunk(q, r + RL * h);
 #pragma unroll
                     for (int p = p0; p < PE; p += 2) {
                         const double2 g = *reinterpret_cast<const double2 *>(rowp + p);
@@ -291,7 +295,7 @@ __device__ __forceinline__ bool tile_solve(const DevJob &J, const DevPlan &P, do
             for (int t = 0; t < XN; ++t) {
                 if (L * t > CL * p0 + CL - 1) continue;
                 if (l + L * t < k) {
-                    const double q = U[at[t].x + s * at[t].y + (s & at[t].z) + p0];
+                    const double q = U[at[t].x + B.chunk(at[t], s) + p0];
                     if (nza) xa[t] = __dsub_rn(xa[t], __dmul_rn(va, q));
                     if (ORD && nzb) xb[t] = __dsub_rn(xb[t], __dmul_rn(vb, q));
                 }

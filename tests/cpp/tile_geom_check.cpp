@@ -42,11 +42,11 @@ static void geometry() {
         own(row + T::pivot(a), i);
         own(row + T::pivot(a) + 1, i);
         // the table form of the same addresses
-        const int x = row - (a & ~1), y = T::chunk(1, a), z = T::cs(a) % 16 == 8 ? 2 : 0;
+        const int x = row - (a & ~1), y = T::spread(a), z = T::mask(a), w = T::shift(a);
         for (int k = i; k < T::NC; ++k)
-            CHECK(x + (k % T::CL) * y + (k % T::CL & z) + k / T::CL ==
+            CHECK(x + (k % T::CL) * y + ((k % T::CL & z) >> w) + k / T::CL ==
                   row + T::chunk(k % T::CL, a) + k / T::CL - (a & ~1));
-        // the four chunks' 16-byte words of one position, on different banks
+        // the chunks' 16-byte words of one position, on different banks
         for (int c = 0; c < T::CL; ++c)
             for (int d = 0; d < c; ++d) CHECK((T::chunk(c, a) - T::chunk(d, a)) / 2 % 8 != 0);
     }
@@ -140,7 +140,7 @@ int main() {
     geometry<TileGeom<48, 4, 4, 6>>();
     geometry<TileGeom<52, 4, 4, 4>>();
     geometry<TileGeom<56, 4, 4, 4>>();
-    geometry<TileGeom<64, 4, 4, 4>>();
+    geometry<TileGeom<64, 8, 4, 4>>();
     square<CokGeom<8, 4, 1>>();
     square<CokGeom<12, 4, 1>>();
     square<CokGeom<16, 4, 2>>();
