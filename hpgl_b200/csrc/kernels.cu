@@ -63,10 +63,48 @@ __global__ void __launch_bounds__(256) k_search_template(DevJob J, DevPlan P) {
 // cut.  Each round scans left from L_{b-1}+1 up to R_{b-1} and right from
 // R_{b-1}-1 down to L_{b-1}; earlier rounds' swaps only ever turn positions
 // at or beyond those bounds into stoppers, which yields the same
-// min(L_m, R_{m-1}).  Ranges up to PAR_PARTITION_MIN elements partition on
-// lane 0.
-constexpr int PAR_PARTITION_MIN = 64;
+// min(L_m, R_{m-1}).  A range of up to 64 elements is one round of two
+// elements a lane (warp_partition64).
 constexpr int SORT_STACK = 72;
+constexpr int TAIL_MAX = 64 + 16;        // positions the final insertion sort reaches
+constexpr int SORT_BUF = TAIL_MAX + 32;  // doubles of scratch a warp
+
+// sort_partition of [pivot + 1, hi), hi - pivot <= 64, pivot the element
+// before the range: the stoppers' ranks come from two 64-bit masks, their
+// positions by rank through lbuf / rbuf (64 each).
+__device__ int warp_partition64(SortArr &a, int pivot, int hi, int *lbuf, int *rbuf, int lane) {
+    const int m = hi - pivot;  // positions pivot + 0 (the pivot) .. pivot + m - 1
+    const double pk = a.key[pivot];
+    bool lst[2], rst[2];
+    unsigned lb[2], rb[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int e = lane + 32 * t;
+        const double k = e < m ? a.key[pivot + e] : 0.0;
+        lst[t] = e > 0 && e < m && !(k > pk);
+        rst[t] = e < m && !(pk > k);
+        lb[t] = __ballot_sync(FULL_MASK, lst[t]);
+        rb[t] = __ballot_sync(FULL_MASK, rst[t]);
+    }
+    const unsigned below = (1u << lane) - 1, above = ~below & ~(1u << lane);
+    const int nl = __popc(lb[0]) + __popc(lb[1]), nr = __popc(rb[0]) + __popc(rb[1]);
+    if (lst[0]) lbuf[__popc(lb[0] & below)] = pivot + lane;
+    if (lst[1]) lbuf[__popc(lb[0]) + __popc(lb[1] & below)] = pivot + lane + 32;
+    if (rst[0]) rbuf[__popc(rb[1]) + __popc(rb[0] & above)] = pivot + lane;
+    if (rst[1]) rbuf[__popc(rb[1] & above)] = pivot + lane + 32;
+    __syncwarp();
+    int pairs = 0;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int e = lane + 32 * t;
+        const bool pair = e < nl && e < nr && lbuf[e] < rbuf[e];  // a prefix of the ranks
+        if (pair) a.swap(lbuf[e], rbuf[e]);
+        pairs += __popc(__ballot_sync(FULL_MASK, pair));
+    }
+    const int lm = pairs < nl ? lbuf[pairs] : INT_MAX, rm = pairs > 0 ? rbuf[pairs - 1] : INT_MAX;
+    __syncwarp();
+    return lm < rm ? lm : rm;
+}
 
 __device__ int warp_partition(SortArr &a, int lo, int hi, int pivot, int *lbuf, int *rbuf, int lane) {
     const double pk = a.key[pivot];
@@ -120,18 +158,18 @@ struct SortFrame {
     int lo, hi, depth;
 };
 
-// reference_sort_prefix driven by a whole warp: control flow is uniform,
-// lane 0 does the median-of-three, small partitions, heap sorts and the final
-// insertion sort, the warp does the long partitions.  `stack` holds
-// SORT_STACK frames, `lbuf`/`rbuf` 32 positions each (shared memory).
-__device__ bool warp_reference_sort_prefix(SortArr &a, int n, int k, int lane, SortFrame *stack, int *lbuf,
-                                           int *rbuf) {
-    if (n <= 1) return true;
+// The partitioning half of reference_sort_prefix driven by a whole warp:
+// control flow is uniform, lane 0 does the median-of-three and heap sorts, the
+// warp the partitions.  Afterwards every position below k lies in a part of
+// at most 16 elements, or in a sorted one, as the reference's sort leaves it
+// for its final insertion sort.  `stack` holds SORT_STACK frames, `lbuf` and
+// `rbuf` 64 positions each (shared memory).
+__device__ bool warp_reference_parts(SortArr &a, int n, int k, int lane, SortFrame *stack, int *lbuf, int *rbuf) {
+    if (n <= 16) return true;
     if (k > n) k = n;
     int sp = 0;
     if (lane == 0) stack[0] = SortFrame{0, n, 2 * sort_floor_log2(n)};
     ++sp;
-    bool ok = true;
     while (sp > 0) {
         __syncwarp();
         const SortFrame f = stack[--sp];
@@ -146,20 +184,10 @@ __device__ bool warp_reference_sort_prefix(SortArr &a, int n, int k, int lane, S
             const int mid = lo + (hi - lo) / 2;
             if (lane == 0) sort_median_to_first(a, lo, lo + 1, mid, hi - 1);
             __syncwarp();
-            int cut;
-            if (hi - lo > PAR_PARTITION_MIN) {
-                cut = warp_partition(a, lo + 1, hi, lo, lbuf, rbuf, lane);
-            } else {
-                int c0 = 0;
-                if (lane == 0) c0 = sort_partition(a, lo + 1, hi, lo);
-                cut = __shfl_sync(FULL_MASK, c0, 0);
-            }
+            const int cut = hi - lo <= 64 ? warp_partition64(a, lo, hi, lbuf, rbuf, lane)
+                                          : warp_partition(a, lo + 1, hi, lo, lbuf, rbuf, lane);
             if (cut < k) {
-                if (sp >= SORT_STACK) {
-                    ok = false;
-                    sp = 0;
-                    break;
-                }
+                if (sp >= SORT_STACK) return false;
                 __syncwarp();
                 if (lane == 0) stack[sp] = SortFrame{cut, hi, depth};
                 ++sp;
@@ -168,18 +196,35 @@ __device__ bool warp_reference_sort_prefix(SortArr &a, int n, int k, int lane, S
         }
     }
     __syncwarp();
-    if (!ok) return false;
-    if (lane == 0) {
-        const int end = (k + 16 < n) ? k + 16 : n;
-        if (n > 16) {
-            sort_insertion(a, 0, 16);
-            for (int i = 16; i < end; ++i) sort_linear_insert(a, i);
-        } else {
-            sort_insertion(a, 0, n);
-        }
+    return true;
+}
+
+// The final insertion sort of reference_sort_prefix and the first k indices of
+// its result, in `out`.  An insertion sort is stable and here moves elements
+// within their part of at most 16 only, so the place of position i is i, plus
+// the later elements before it, less the earlier elements it is before, among
+// its 15 neighbours on either side: counted for 32 positions at once where
+// lane 0 moved them one after another.  s: SORT_BUF doubles.
+__device__ void warp_sort_tail(const SortArr &a, int n, int k, double *s, int *out, int lane) {
+    const int end = k + 16 < n ? k + 16 : n;
+    for (int i = lane; i < end + 32; i += 32) {
+        // 16 sentinels either side: never before, never after
+        double v = i < 16 ? __longlong_as_double(0x7ff0000000000000LL) : __longlong_as_double(0xfff0000000000000LL);
+        if (i >= 16 && i < end + 16) v = a.key[i - 16];
+        s[i] = v;
     }
     __syncwarp();
-    return true;
+    for (int i = lane; i < end; i += 32) {
+        const double v = s[i + 16];
+        int at = i;
+#pragma unroll 5
+        for (int d = 1; d < 16; ++d) {
+            if (s[i + 16 + d] > v) ++at;
+            if (s[i + 16 - d] < v) --at;
+        }
+        if (at < k && at < n) out[at] = a.idx[i];
+    }
+    __syncwarp();
 }
 
 // ---------------------------------------------------------------------------
@@ -189,7 +234,12 @@ __device__ bool warp_reference_sort_prefix(SortArr &a, int n, int k, int lane, S
 // keeps those with covariance above C(0)/100 (order-preserving ballot
 // compaction), then the warp orders them exactly as the reference's
 // std::sort does — as far as the first max_neighbours positions, which become
-// the list.
+// the list.  Bound by instruction issue and the latency of the candidates'
+// scratch (L1, L2): parts of up to 64 elements and the final insertion sort
+// were lane 0's, a chain of dependent accesses each; as warp-wide counts and
+// ballots LVM 512x512x32 searches in 23.6 ms (35.0), OK 61x64x12 with 60
+// neighbours in 0.40 (1.32), OK 88x88x20 with 2 900 candidates a node, where
+// the long partitions remain, in 8.7 (10.0).
 constexpr int CLUSTER_WARPS = 4;
 constexpr int CLUSTER_CHUNK = 16;  // nodes a warp takes from the counter at a time
 
@@ -197,7 +247,9 @@ constexpr int CLUSTER_CHUNK = 16;  // nodes a warp takes from the counter at a t
 __global__ void __launch_bounds__(CLUSTER_WARPS * 32, 16) k_search_cluster(DevJob J, DevPlan P, double *scratch_key,
                                                                       int *scratch_idx, int n_warps_total) {
     __shared__ SortFrame s_stack[CLUSTER_WARPS][SORT_STACK];
-    __shared__ int s_lbuf[CLUSTER_WARPS][32], s_rbuf[CLUSTER_WARPS][32];
+    // the partitions' positions by rank, then the tail's keys
+    __shared__ double s_buf[CLUSTER_WARPS][SORT_BUF];
+    static_assert(SORT_BUF * sizeof(double) >= 128 * sizeof(int), "room for both position lists");
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -223,46 +275,48 @@ __global__ void __launch_bounds__(CLUSTER_WARPS * 32, 16) k_search_cluster(DevJo
             const int cx = (int)(x / P.crx), cy = (int)(y / P.cry), cz = (int)(z / P.crz);
             int n = 0;
             for (int k = cz - 1; k <= cz + 1; ++k)
-                for (int j = cy - 1; j <= cy + 1; ++j)
-                    for (int i = cx - 1; i <= cx + 1; ++i) {
-                        if (i < 0 || j < 0 || k < 0 || i > P.mx || j > P.my || k > P.mz) continue;
-                        const long long bi = ((long long)k * P.my + j) * P.mx + i;
-                        const int s0 = P.bucket_start[bi], s1 = P.bucket_start[bi + 1];
-                        for (int base = s0; base < s1; base += 32) {
-                            const int p = base + lane;
-                            bool keep = false;
-                            double key = 0;
-                            int cand = 0;
-                            if (p < s1) {
-                                cand = P.bucket_nodes[p];
-                                int qx, qy, qz;
-                                node_xyz(J, cand, qx, qy, qz);
-                                key = cov_at(P, qx - x, qy - y, qz - z, J.err);
-                                keep = key > thr;
-                            }
-                            const uint32_t bal = __ballot_sync(FULL_MASK, keep);
-                            const int pos = n + __popc(bal & ((1u << lane) - 1));
-                            if (keep) {
-                                if (pos < cap) {
-                                    keys[pos] = key;
-                                    idxs[pos] = cand;
-                                } else {
-                                    atomicOr(J.err, DERR_CAND_CAPACITY);
-                                }
-                            }
-                            n += __popc(bal);
+                for (int j = cy - 1; j <= cy + 1; ++j) {
+                    if (j < 0 || k < 0 || j > P.my || k > P.mz) continue;
+                    // the boxes of one row follow one another in the buckets
+                    const int i0 = max(cx - 1, 0), i1 = min(cx + 1, P.mx);
+                    const long long bi = ((long long)k * P.my + j) * P.mx;
+                    const int s0 = P.bucket_start[bi + i0], s1 = P.bucket_start[bi + i1 + 1];
+                    for (int base = s0; base < s1; base += 32) {
+                        const int p = base + lane;
+                        bool keep = false;
+                        double key = 0;
+                        int cand = 0;
+                        if (p < s1) {
+                            cand = P.bucket_nodes[p];
+                            int qx, qy, qz;
+                            node_xyz(J, cand, qx, qy, qz);
+                            key = cov_at(P, qx - x, qy - y, qz - z, J.err);
+                            keep = key > thr;
                         }
+                        const uint32_t bal = __ballot_sync(FULL_MASK, keep);
+                        const int pos = n + __popc(bal & ((1u << lane) - 1));
+                        if (keep) {
+                            if (pos < cap) {
+                                keys[pos] = key;
+                                idxs[pos] = cand;
+                            } else {
+                                atomicOr(J.err, DERR_CAND_CAPACITY);
+                            }
+                        }
+                        n += __popc(bal);
                     }
+                }
             if (n > cap) n = cap;
             __syncwarp();
             {
                 // only the first max_neighbours positions of the reference's sort are used
                 SortArr a{keys, idxs};
-                if (!warp_reference_sort_prefix(a, n, P.nmax, lane, s_stack[wib], s_lbuf[wib], s_rbuf[wib]) && lane == 0)
+                int *lbuf = reinterpret_cast<int *>(s_buf[wib]);
+                if (!warp_reference_parts(a, n, P.nmax, lane, s_stack[wib], lbuf, lbuf + 64) && lane == 0)
                     atomicOr(J.err, DERR_SORT_STACK);
+                warp_sort_tail(a, n, P.nmax, s_buf[wib], J.nb + (long long)node * P.nmax, lane);
             }
             const int cnt = n < P.nmax ? n : P.nmax;
-            for (int i = lane; i < cnt; i += 32) J.nb[(long long)node * P.nmax + i] = idxs[i];
             if (lane == 0) J.nbcount[node] = cnt;
             __syncwarp();
         }
