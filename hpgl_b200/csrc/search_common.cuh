@@ -1,6 +1,8 @@
 // Template search of one 32-node x-segment, shared by the search kernel and
 // the fused search+solve kernels.
 #pragma once
+#include <climits>
+
 #include "device_common.cuh"
 
 namespace hpgl_b200 {
@@ -44,19 +46,30 @@ __device__ __forceinline__ int template_segment(const DevJob &J, const DevPlan &
     int cnt = 0;
     int *out = J.nb + (long long)node * nmax;
     const uint32_t *bits = J.bits;
+    auto entry = [&](int t) {
+        // past the end: a row outside every grid
+        return (unsigned)t < (unsigned)P.tmpl_len ? __ldg(&P.tmpl[t]) : make_int4(0, INT_MIN / 2, 0, 0);
+    };
+    auto window = [&](const int4 &e) {
+        const int yy = y + e.y, zz = z + e.z;
+        if ((unsigned)yy >= (unsigned)J.ny || (unsigned)zz >= (unsigned)J.nz) return 0u;
+        const uint32_t *rp = bits + ((long long)zz * J.ny + yy) * P.wpr + seg + (e.x >> 5);
+        return __funnelshift_r(__ldg(rp), __ldg(rp + 1), e.x & 31);
+    };
+    // The windows are loaded one chunk ahead of their use, the entries two: a
+    // segment is one warp's chain of chunks, and a small grid has too few
+    // segments to hide two dependent loads a chunk (OK 50x50x20: search 52 ->
+    // 44 us; SK 256x256x64, which has enough, 2.84 -> 2.72 ms).
+    int4 e = entry(lane);
+    uint32_t next_w = window(e);
+    int next_delta = e.w;
+    e = entry(lane + 32);
     for (int tb = 0; tb < P.tmpl_len && active; tb += 32) {
-        const int t = tb + lane;
-        uint32_t w = 0;
-        int delta = 0;
-        if (t < P.tmpl_len) {
-            const int4 e = __ldg(&P.tmpl[t]);
-            delta = e.w;
-            const int yy = y + e.y, zz = z + e.z;
-            if ((unsigned)yy < (unsigned)J.ny && (unsigned)zz < (unsigned)J.nz) {
-                const uint32_t *rp = bits + ((long long)zz * J.ny + yy) * P.wpr + seg + (e.x >> 5);
-                w = __funnelshift_r(__ldg(rp), __ldg(rp + 1), e.x & 31);
-            }
-        }
+        uint32_t w = next_w;
+        const int delta = next_delta;
+        next_w = window(e);
+        next_delta = e.w;
+        e = entry(tb + 64 + lane);
         w &= active;
         dsm[lane] = delta;
         uint32_t hits = transpose32(w, lane);
