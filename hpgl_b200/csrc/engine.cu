@@ -620,8 +620,19 @@ static void parallel_copy(void *dst, const void *src, size_t bytes) {
     }, 4LL << 20);
 }
 
-// staging: pinned host memory of at least the main outputs' size (the
-// estimate or codes and the mask), or null for direct copies.
+// The main outputs (the estimate or codes and the mask) to pinned host memory.
+static void stage_outputs(const JobState &S, cudaStream_t s, char *staging) {
+    const Arena &A = S.ar;
+    const size_t n = (size_t)S.size;
+    const bool cont = kind_is_cont(S.job.kind);
+    const size_t main_bytes = cont ? n * 4 : n;
+    const void *dev_main = cont ? (const void *)at<float>(S, A.o_out_values) : (const void *)at<uint8_t>(S, A.o_out_codes);
+    CUDA_CHECK(cudaMemcpyAsync(staging, dev_main, main_bytes, cudaMemcpyDeviceToHost, s));
+    CUDA_CHECK(cudaMemcpyAsync(staging + main_bytes, at<uint8_t>(S, A.o_out_mask), n, cudaMemcpyDeviceToHost, s));
+}
+
+// staging: the main outputs as stage_outputs left them (the stream has been
+// waited for since), or null for direct copies.
 static void download(const JobState &S, hpgl_b200_result_t &res, const Counters &cnt, cudaStream_t s,
                      char *staging = nullptr) {
     const hpgl_b200_job_t &job = S.job;
@@ -646,10 +657,7 @@ static void download(const JobState &S, hpgl_b200_result_t &res, const Counters 
     void *out_main = cont ? (void *)res.out_values : (void *)res.out_codes;
     const size_t main_bytes = cont ? n * 4 : n;
     const void *dev_main = cont ? (const void *)at<float>(S, A.o_out_values) : (const void *)at<uint8_t>(S, A.o_out_codes);
-    if (staging) {
-        CUDA_CHECK(cudaMemcpyAsync(staging, dev_main, main_bytes, cudaMemcpyDeviceToHost, s));
-        CUDA_CHECK(cudaMemcpyAsync(staging + main_bytes, at<uint8_t>(S, A.o_out_mask), n, cudaMemcpyDeviceToHost, s));
-    } else {
+    if (!staging) {
         CUDA_CHECK(cudaMemcpyAsync(out_main, dev_main, main_bytes, cudaMemcpyDeviceToHost, s));
         CUDA_CHECK(cudaMemcpyAsync(res.out_mask, at<uint8_t>(S, A.o_out_mask), n, cudaMemcpyDeviceToHost, s));
     }
@@ -665,7 +673,7 @@ static void download(const JobState &S, hpgl_b200_result_t &res, const Counters 
         CUDA_CHECK(cudaMemcpy2DAsync(res.weights, (size_t)res.nb_stride * 8, at<double>(S, A.o_weights), wn * 8,
                                      wn * 8, slots, cudaMemcpyDeviceToHost, s));
     }
-    CUDA_CHECK(cudaStreamSynchronize(s));
+    if (!staging || res.status || res.variance || res.probs || res.weights) CUDA_CHECK(cudaStreamSynchronize(s));
     if (staging) {
         parallel_copy(out_main, staging, main_bytes);
         parallel_copy(res.out_mask, staging + main_bytes, n);
@@ -683,6 +691,7 @@ static void download(const JobState &S, hpgl_b200_result_t &res, const Counters 
 
 struct SyncContext {
     cudaStream_t stream = nullptr;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;  // around a job's device pass
     char *arena = nullptr;
     size_t cap = 0;
     char *inputs = nullptr;   // the job's inputs, uploaded while it is planned
@@ -703,6 +712,8 @@ static SyncContext &sync_ctx() {
         ensure_device();
         auto *nc = new SyncContext();
         CUDA_CHECK(cudaStreamCreateWithFlags(&nc->stream, cudaStreamNonBlocking));
+        CUDA_CHECK(cudaEventCreate(&nc->e0));
+        CUDA_CHECK(cudaEventCreate(&nc->e1));
         c = nc;
     }
     return *c;
@@ -825,8 +836,9 @@ void run_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res) {
         sync_arena(C, S.ar.total - in_total);
         S.in_base = C.inputs;
         S.rest = C.arena;
+        // The pass follows on the same stream, with no wait for the uploads:
+        // a copy from pageable memory returns once its source has been read.
         upload_rest(S, C.stream);
-        CUDA_CHECK(cudaStreamSynchronize(C.stream));
         res.ms_h2d = ms_since(t1);
     } else {
         auto t1 = std::chrono::steady_clock::now();
@@ -836,20 +848,17 @@ void run_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res) {
         CUDA_CHECK(cudaStreamSynchronize(C.stream));
         res.ms_h2d = ms_since(t1);
     }
-    cudaEvent_t e0, e1;
-    CUDA_CHECK(cudaEventCreate(&e0));
-    CUDA_CHECK(cudaEventCreate(&e1));
-    CUDA_CHECK(cudaEventRecord(e0, C.stream));
+    CUDA_CHECK(cudaEventRecord(C.e0, C.stream));
     const bool want_nb = res.nb_count || res.nb_index;
     device_pass(S, C.stream, nullptr, [&](const Group &g) {
         if (want_nb) download_neighbours(S, g, res, C.stream);
     });
-    CUDA_CHECK(cudaEventRecord(e1, C.stream));
+    CUDA_CHECK(cudaEventRecord(C.e1, C.stream));
+    // one wait for the pass, its counters and its staged outputs
+    if (staging) stage_outputs(S, C.stream, staging);
     Counters cnt = read_counters(S, C.stream);
     float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    cudaEventElapsedTime(&ms, C.e0, C.e1);
     res.ms_device = ms;
     auto t2 = std::chrono::steady_clock::now();
     download(S, res, cnt, C.stream, staging);
