@@ -438,6 +438,8 @@ static void upload_rest(JobState &S, cudaStream_t s) {
             d.pk = OffsetPack(reach, t3);
         }
         d.c0 = P.c0;
+        std::copy(P.reach_t, P.reach_t + 9, d.reach_t);
+        d.reach_limit = P.reach_limit;
         d.bucket_start = at<int>(S, g.o_bstart);
         d.bucket_nodes = at<int>(S, g.o_bnodes);
         d.bucket_clean = at<uint8_t>(S, g.o_bclean);

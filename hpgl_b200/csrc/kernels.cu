@@ -237,11 +237,29 @@ __device__ void warp_sort_tail(const SortArr &a, int n, int k, double *s, int *o
 // the list.  Bound by instruction issue and the latency of the candidates'
 // scratch (L1, L2): parts of up to 64 elements and the final insertion sort
 // were lane 0's, a chain of dependent accesses each; as warp-wide counts and
-// ballots LVM 512x512x32 searches in 23.6 ms (35.0), OK 61x64x12 with 60
+// ballots LVM 512x512x32 searches in 24.4 ms (35.0), OK 61x64x12 with 60
 // neighbours in 0.40 (1.32), OK 88x88x20 with 2 900 candidates a node, where
-// the long partitions remain, in 8.7 (10.0).
+// the long partitions remain, in 8.7 (10.0).  Where most candidates of the 27
+// boxes fail the filter their reads of the table are the traffic: those beyond
+// the model's reach are dropped by their offset (OK 251x213x51, 13 600
+// candidates of which 3 400 pass: 316 -> 274 ms), and the next candidates are
+// read a chunk ahead (258).  LVM's truncated model, whose range test drops
+// most anyway, pays 0.5 ms for it.
 constexpr int CLUSTER_WARPS = 4;
-constexpr int CLUSTER_CHUNK = 16;  // nodes a warp takes from the counter at a time
+// |reach_t d|^2 (Plan): beyond reach_limit the covariance is at most C(0)/100.
+__device__ __forceinline__ float reach2(const DevPlan &P, float dx, float dy, float dz) {
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const float u = P.reach_t[3 * i] * dx + P.reach_t[3 * i + 1] * dy + P.reach_t[3 * i + 2] * dz;
+        q += u * u;
+    }
+    return q;
+}
+// Nodes a warp takes from the counter at a time: at most this many, fewer where
+// a small grid would leave warps without any (OK 61x64x12: 0.40 -> 0.19 ms with
+// 2 in place of 16).
+constexpr int CLUSTER_CHUNK = 16;
 
 // 16 blocks a SM (32 registers): the engine launches 64 warps a SM
 __global__ void __launch_bounds__(CLUSTER_WARPS * 32, 16) k_search_cluster(DevJob J, DevPlan P, double *scratch_key,
@@ -258,15 +276,17 @@ __global__ void __launch_bounds__(CLUSTER_WARPS * 32, 16) k_search_cluster(DevJo
     double *keys = scratch_key + (long long)gw * cap;
     int *idxs = scratch_idx + (long long)gw * cap;
     const double thr = P.c0 / 100;
-    // warps take CLUSTER_CHUNK consecutive nodes at a time from a counter:
+    const unsigned below = (1u << lane) - 1;
+    // warps take a few consecutive nodes at a time from a counter:
     // clusterizer-path nodes sit in sparse regions, so a fixed share would
     // leave some warps most of them
+    const int take = (int)min((long long)CLUSTER_CHUNK, max(1LL, (long long)J.size / (2 * n_warps_total)));
     while (true) {
         int chunk = 0;
-        if (lane == 0) chunk = atomicAdd(J.node_next, CLUSTER_CHUNK);
+        if (lane == 0) chunk = atomicAdd(J.node_next, take);
         chunk = __shfl_sync(FULL_MASK, chunk, 0);
         if (chunk >= J.size) break;
-        const int chunk_end = (int)min((long long)chunk + CLUSTER_CHUNK, (long long)J.size);
+        const int chunk_end = (int)min((long long)chunk + take, (long long)J.size);
         for (int node = chunk; node < chunk_end; ++node) {
             if (!node_needs_kriging(J, node)) continue;
             int x, y, z;
@@ -281,20 +301,25 @@ __global__ void __launch_bounds__(CLUSTER_WARPS * 32, 16) k_search_cluster(DevJo
                     const int i0 = max(cx - 1, 0), i1 = min(cx + 1, P.mx);
                     const long long bi = ((long long)k * P.my + j) * P.mx;
                     const int s0 = P.bucket_start[bi + i0], s1 = P.bucket_start[bi + i1 + 1];
+                    int next = s0 + lane < s1 ? __ldg(P.bucket_nodes + s0 + lane) : -1;
                     for (int base = s0; base < s1; base += 32) {
-                        const int p = base + lane;
+                        const int cand = next;
+                        next = base + 32 + lane < s1 ? __ldg(P.bucket_nodes + base + 32 + lane) : -1;
                         bool keep = false;
                         double key = 0;
-                        int cand = 0;
-                        if (p < s1) {
-                            cand = P.bucket_nodes[p];
-                            int qx, qy, qz;
-                            node_xyz(J, cand, qx, qy, qz);
-                            key = cov_at(P, qx - x, qy - y, qz - z, J.err);
-                            keep = key > thr;
+                        if (cand >= 0) {
+                            int dx, dy, dz;
+                            node_xyz(J, cand, dx, dy, dz);
+                            dx -= x;
+                            dy -= y;
+                            dz -= z;
+                            if (!(reach2(P, (float)dx, (float)dy, (float)dz) > P.reach_limit)) {
+                                key = cov_at(P, dx, dy, dz, J.err);
+                                keep = key > thr;
+                            }
                         }
                         const uint32_t bal = __ballot_sync(FULL_MASK, keep);
-                        const int pos = n + __popc(bal & ((1u << lane) - 1));
+                        const int pos = n + __popc(bal & below);
                         if (keep) {
                             if (pos < cap) {
                                 keys[pos] = key;

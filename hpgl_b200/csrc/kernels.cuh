@@ -36,6 +36,7 @@ struct DevPlan {
     const int *bucket_start;
     const int *bucket_nodes;
     const uint8_t *bucket_clean;
+    float reach_t[9], reach_limit;  // offsets that can pass the covariance filter (Plan)
     double crx, cry, crz;
     int mx, my, mz;
     int max_candidates;

@@ -205,6 +205,27 @@ double CovModel::operator()(double vx, double vy, double vz) const {
     }
 }
 
+// The clusterizer keeps candidates of C(d) > C(0)/100.  C falls with
+// h = |T d|, so only h below the distance where the model falls to a hundredth
+// can pass.  The limit has room for the roundings: 1e-3 of h for the model's,
+// and for |T d| in single precision, whose terms may cancel, 1e-6 of the
+// largest sum of their magnitudes (a sum of three products is off by at most 4
+// roundings of 6e-8 each, the coefficients' included, per component).
+static void cov_reach(const CovModel &cov, const int n[3], float t[9], float &limit) {
+    double magnitude = 0;
+    for (int i = 0; i < 9; ++i) {
+        t[i] = (float)cov.t[i];
+        magnitude += fabs(cov.t[i]) * n[i % 3];
+    }
+    limit = INFINITY;
+    if (!(cov.sill - cov.nugget > 0) || !(cov.range0 > 0)) return;
+    // spherical: 1 - 1.5 r + 0.5 r^3 = 0.01 at r = 0.9172; exponential: exp(-3 r);
+    // Gaussian: exp(-3 r^2)
+    const double r = cov.type == 2 ? sqrt(log(100.0) / 3) : cov.type == 1 ? log(100.0) / 3 : 0.918;
+    const double h = cov.range0 * r * 1.001 + 0.001 + 1e-6 * magnitude;
+    limit = (float)(h * h);
+}
+
 void validate_params(const KrigingParams &p, int kind) {
     if (p.cov_type < 0 || p.cov_type > 2) throw std::invalid_argument("covariance type must be 0, 1 or 2");
     for (int i = 0; i < 3; ++i) {
@@ -539,6 +560,7 @@ void build_plan(Plan &P, int kind, int nx, int ny, int nz, const KrigingParams &
                        [&](int x, int y, int z) { return cov((double)x, (double)y, (double)z); });
     }
     P.c0 = c0;
+    cov_reach(cov, n3, P.reach_t, P.reach_limit);
     lap("table");
 
     // ---- informed-bit rows for the device template search ----

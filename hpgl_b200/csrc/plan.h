@@ -85,6 +85,11 @@ struct Plan {
     RawVector<double> table;
     double c0 = 0;  // C(0)
 
+    // Offsets d whose covariance can exceed C(0)/100: |reach_t d|^2 <= reach_limit,
+    // with room for its evaluation in single precision (cov_reach).
+    float reach_t[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    float reach_limit = 0;
+
     // clusterizer (clusterizer.cpp:52-184)
     double cl_r[3] = {0, 0, 0};
     int mx = 0, my = 0, mz = 0;

@@ -34,3 +34,25 @@ def test_lists_match_std_sort(native_lib, points, nmax):
     ok, msg = neighbour_lists_equal(ref, got, sr, sr, ref["cap"], got["cap"])
     assert ok, msg
     assert f32_bits_equal(got["out"], ref["out"])
+
+
+@pytest.mark.parametrize("kind", ["ok", "sk"])
+@pytest.mark.parametrize("cov", [0, 1, 2])
+@pytest.mark.parametrize("ranges", [(9, 9, 9), (12, 5, 3), (3, 200, 1), (0.004, 5, 5), (5000, 2, 2)])
+def test_candidates_within_reach(native_lib, kind, cov, ranges):
+    # the candidates that are dropped before their covariance is read are
+    # those it would drop, at skewed and extreme anisotropies
+    rng = np.random.default_rng(cov)
+    shape = (37, 33, 9)
+    size = int(np.prod(shape))
+    mask = (rng.random(size) < 0.02).astype(np.uint8)
+    values = np.where(mask > 0, rng.standard_normal(size), -99).astype(np.float32)
+    p = W.cov_params(cov, ranges, angles=(25, 10, 5), sill=1.0, nugget=0.1, radii=(30, 31, 32), max_neighbours=20)
+    job = dict(kind=kind, shape=shape, mask=mask, values=values, params=[p], sk_mean=0.1)
+    ref = O.run(job, kind=kind)
+    got = N.krige(job, precision="fp64", kind=kind, dumps=True)
+    sr = np.nonzero(ref["status"] >= 0)[0]
+    assert np.array_equal(ref["status"], got["status"])
+    ok, msg = neighbour_lists_equal(ref, got, sr, sr, ref["cap"], got["cap"])
+    assert ok, msg
+    assert f32_bits_equal(got["out"], ref["out"])
