@@ -8,11 +8,12 @@ azimuth 30, sill 1, nugget 0.05, radii (80,40,16), 32 neighbours, SK mean 0
 (hpgl_b200.workloads.sk_ok_256x256x64) — every uninformed node kriged once.
 Metric: kriged nodes/s.
 
-* ``value``: FP32 factorisation + FP64 refinement, device-resident (inputs
-  in HBM before the timed region; each step re-runs search, covariance
-  build, solve and estimate), CUDA events on the library's stream, 256 MiB
-  written between steps to flush L2; whole job = all ranks' nodes / max rank
-  time.  ``fp64`` holds the same for the bit-exact FP64 path and
+* ``value``: the mixed-precision request, whose systems are solved in FP64 in
+  the reference's operation order since those solves are the faster ones,
+  device-resident (inputs in HBM before the timed region; each step re-runs
+  search, covariance build, solve and estimate), CUDA events on the library's
+  stream, 256 MiB written between steps to flush L2; whole job = all ranks'
+  nodes / max rank time.  ``fp64`` holds the same for an FP64 request and
   ``mixed_vs_fp64`` their ratio.
 * ``e2e``: the same metric through the public C ABI (hpgl_b200_krige) from
   host buffers: planning, host->device copies, device work and device->host
@@ -289,9 +290,9 @@ def main():
     h2d = size * 4 + size * 1
     d2h = size * 4 + size * 1
 
-    # Per-result error of the mixed path against the FP64 path (bit-identical
-    # to the reference's arithmetic): every kriged node's estimate and
-    # kriging variance, untimed.
+    # Per-result error of the mixed request against the FP64 one
+    # (bit-identical to the reference's arithmetic): every kriged node's
+    # estimate and kriging variance, untimed.
     ref64 = N.krige(job, precision="fp64", dumps="variance")
     mix = N.krige(job, precision="mixed", dumps="variance")
     okv = ref64["status"] == 0
@@ -307,11 +308,12 @@ def main():
     del ref64, mix
 
     # Roofline of the dominant kernel (the solve): algorithmic flops per
-    # launch / CUDA-event duration, against the FP32 CUDA-core rate measured
+    # launch / CUDA-event duration, against the FP64 CUDA-core rate measured
     # here by an FMA-loop kernel timed alone (hpgl_b200_fma_peak; the
-    # measured-peaks file holds HBM and bf16-tensor figures only).
-    peak_fp32 = N.fma_peak("mixed")
-    peak_fp64 = N.fma_peak("fp64")
+    # measured-peaks file holds HBM and bf16-tensor figures only).  The solve
+    # rounds every product and sum apart, as the reference does, so half the
+    # fused rate is its ceiling.
+    peak = N.fma_peak("fp64")
     achieved = flops / (info_m["ms_top_kernel"] / 1000.0) / 1e12
     achieved64 = flops / (info_f["ms_top_kernel"] / 1000.0) / 1e12
     traffic = None
@@ -321,12 +323,12 @@ def main():
         traffic = tj["dram_bytes_per_launch_128x128x32"] * kriged / tj["systems_128x128x32"]
     except (OSError, KeyError, ValueError):
         pass
-    roofline = {"kernel": info_m["top_kernel"], "bound": "fp32", "achieved": achieved, "peak": peak_fp32,
-                "unit": "TFLOP/s", "frac": achieved / peak_fp32, "traffic": traffic, "traffic_unit": "bytes/launch",
-                "peak_source": "measured FP32 CUDA-core rate, FMA-loop kernel timed alone (hpgl_b200_fma_peak)",
+    roofline = {"kernel": info_m["top_kernel"], "bound": "fp64", "achieved": achieved, "peak": peak,
+                "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic, "traffic_unit": "bytes/launch",
+                "peak_source": "measured FP64 CUDA-core rate, FMA-loop kernel timed alone (hpgl_b200_fma_peak)",
                 "ms_per_launch": info_m["ms_top_kernel"], "flop_per_launch": flops,
-                "fp64_solve": {"kernel": info_f["top_kernel"], "achieved": achieved64, "peak": peak_fp64,
-                               "frac": achieved64 / peak_fp64, "ms_per_launch": info_f["ms_top_kernel"]}}
+                "fp64_solve": {"kernel": info_f["top_kernel"], "achieved": achieved64, "peak": peak,
+                               "frac": achieved64 / peak, "ms_per_launch": info_f["ms_top_kernel"]}}
 
     # Serving: Poisson streams of mixed OK/SK/IK jobs (grids 32^3 ..
     # 256x256x64, ranges 5-60, 8-64 neighbours) replayed in real time
@@ -370,9 +372,9 @@ def main():
         line = {
             "metric": METRIC, "value": value, "unit": "nodes/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": t_mixed / args.steps, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64", "data": "synthetic",
+            "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
             "config": {"workload": WORKLOAD, "grid": list(job["shape"]), "kriged_nodes_per_step": kriged,
-                       "precision": "fp32 factorisation + fp64 refinement, fp64 re-solve of routed systems",
+                       "precision": "fp64 solves in the reference's operation order (mixed request)",
                        "l2": "256 MiB written between steps", "parallelism": "replicas%d" % world,
                        "launch": tuning, "pass": "one CUDA graph per step"},
             "fp64": {"value": fp64_value, "ms_per_step": t_fp64 / args.steps,

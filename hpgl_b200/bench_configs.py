@@ -6,8 +6,8 @@ ordinary kriging 50x50x20 (12 neighbours), simple and ordinary kriging
 neighbours, one shared system per node: the four variograms are equal),
 LVM kriging 512x512x32 (64 neighbours).  Per case: the device pass (CUDA
 events, inputs in HBM, 256 MiB written between passes, one CUDA-graph
-replay per pass) for the FP32-refined path and for plain FP64, the share
-of systems the mixed path re-solved in FP64, and whole hpgl_b200_krige calls
+replay per pass) for a mixed and for an FP64 request, the share of systems
+the mixed request solved in FP64, and whole hpgl_b200_krige calls
 from host buffers (median of three after one warm-up call).  Unit: kriged systems per second (IK counts a
 system per category, as the reference solves one per category).
 """
@@ -54,7 +54,7 @@ def run(args, root):
     first = cases["ik_200x200x100:ik"]
     line = {
         "metric": "kriged systems/s", "value": first["mixed"]["systems_per_s"], "unit": "systems/s", "n_gpus": 1,
-        "steps": steps, "warmup": warmup, "higher_is_better": True, "dtype": "f32+f64", "data": "synthetic",
+        "steps": steps, "warmup": warmup, "higher_is_better": True, "dtype": "f64", "data": "synthetic",
         "config": {"workload": "ik_200x200x100 (value) and every configuration (cases)",
                    "l2": "256 MiB written between passes"},
         "cases": cases,

@@ -4,9 +4,9 @@ The jobs of hpgl_b200.workloads.serve_stream (40 jobs, seed 5: grids
 log-uniform between 32^3 and 256x256x64, 0.5-3 % informed, spherical /
 exponential / Gaussian variograms with ranges 5-60, 8-64 neighbours, OK / SK
 / 4-category IK), each run alone: the device pass (CUDA events, inputs in
-HBM, one CUDA-graph replay per pass) in the FP32-refined and plain FP64
-precisions, with its search and top-kernel times, the systems solved and the
-share re-solved in FP64.  Shows which jobs the stream's device time goes to.
+HBM, one CUDA-graph replay per pass) for a mixed and for an FP64 request, with
+its search and top-kernel times, the systems solved and the share solved in
+FP64.  Shows which jobs the stream's device time goes to.
 
 ``--job NAME`` keeps one job (e.g. serve_31); ``--crop NXxNYxNZ`` cuts its
 cube to the first NX x NY x NZ cells with the same variogram and search
@@ -58,7 +58,7 @@ def run(args, root):
     total = {prec: sum(r[prec]["ms"] for r in rows) for prec in ("mixed", "fp64")}
     systems = sum(r["mixed"]["systems"] for r in rows)
     print(json.dumps({"metric": "kriged systems/s", "value": systems / (total["mixed"] / 1e3), "unit": "systems/s",
-                      "n_gpus": 1, "steps": steps, "warmup": warmup, "higher_is_better": True, "dtype": "f32+f64",
+                      "n_gpus": 1, "steps": steps, "warmup": warmup, "higher_is_better": True, "dtype": "f64",
                       "data": "synthetic",
                       "config": {"workload": "serving stream jobs, each alone (%d jobs%s%s)" % (
                           len(rows), ", job " + args.job if args.job else "", ", crop " + args.crop if args.crop else "")},

@@ -1129,7 +1129,7 @@ void bench_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res, hpgl_b200_be
     bench.ms_search = search_sum / phase_runs;
     bench.ms_resolve = resolve_sum / phase_runs;
     snprintf(bench.top_kernel, sizeof(bench.top_kernel), "%s",
-             S.cok ? "k_cokriging"
+             S.cok ? (S.groups[0].dp.pk.m != 0 && S.nmax_all <= 48 ? "k_cok_tile" : "k_cokriging")
                    : top_kernel_name(S.nmax_all,
                                      tuning_get(tuning_family(S.nmax_all), S.precision).schedule));
     bench.launches_per_iter = pt.launches;

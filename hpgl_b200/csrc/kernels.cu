@@ -401,7 +401,7 @@ void launch_solve(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_
 
 // ---------------------------------------------------------------------------
 // Speculative sequential simulation: path ranks, commits and admissions (the
-// rounds' kriging is k_sgs_try32 / k_sgs_try64).
+// rounds' kriging is launch_sgs_try32 / launch_sgs_try64 in the solve files).
 
 __global__ void k_sgs_rank_init(DevJob J, int *rank_of) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;

@@ -17,7 +17,7 @@ namespace {
 constexpr int CHAINS = 8;     // independent accumulators per thread
 constexpr int UNROLL = 64;    // multiply-adds per chain per loop trip
 
-// FP32: packed two-wide fused multiply-adds (the form the mixed solve uses),
+// FP32: packed two-wide fused multiply-adds,
 // 2 x CHAINS x UNROLL x iters multiply-adds per thread.
 __global__ void __launch_bounds__(256) k_peak_f32(float *out, int iters, float a, float b) {
     float2 acc[CHAINS];

@@ -260,10 +260,10 @@ int hpgl_get_last_error(void);
    and by hpgl_b200_krige when its own field is -1.
    HPGL_PRECISION_FP64: the reference's FP64 Cholesky in its exact operation
    order — results bit-identical to the reference's.
-   HPGL_PRECISION_MIXED: FP32 factorisation with FP64 iterative refinement;
-   systems whose FP32 pivots fail a threshold, or whose refinement does not
-   converge, are re-solved with the FP64 path.  Masks are identical to the
-   reference's; estimates and variances agree to <= 1e-6 relative.
+   HPGL_PRECISION_MIXED: permits FP32 arithmetic within 1e-6 relative on
+   estimates and variances, with identical masks.  Every system is solved in
+   FP64 in this build, as its FP64 solves are faster than an FP32
+   factorisation with FP64 refinement; the setting selects the launch tuning.
    The default is HPGL_PRECISION_FP64, or the value of the environment
    variable HPGL_B200_PRECISION ("fp64" / "mixed") at library load. */
 #define HPGL_PRECISION_FP64 0
@@ -386,7 +386,7 @@ typedef struct hpgl_b200_bench_t {
     long long systems_fp64;
     double ms_plan;
     double ms_search;             /* average device time of the first group's searches */
-    double ms_resolve;            /* ... and of its FP64 re-solve of routed systems */
+    double ms_resolve;            /* ... and of what follows its solve (nothing in this build) */
 } hpgl_b200_bench_t;
 int hpgl_b200_bench(const hpgl_b200_job_t *job, hpgl_b200_result_t *result, hpgl_b200_bench_t *bench);
 
