@@ -351,6 +351,7 @@ static void build_buckets(Plan &P, int nx, int ny, int nz, const KrigingParams &
     }
     P.bucket_clean.assign(nb, 0);
     P.any_clean = false;
+    P.all_clean = true;
     P.max_candidates = 0;
     // Only boxes that hold grid nodes are ever asked (cx < nx/rx + 1 < mx).
     for (int cz = 0; cz < P.mz; ++cz)
@@ -375,6 +376,8 @@ static void build_buckets(Plan &P, int nx, int ny, int nz, const KrigingParams &
                 if (clean) {
                     P.any_clean = true;
                     P.max_candidates = std::max(P.max_candidates, cand);
+                } else {
+                    P.all_clean = false;
                 }
             }
 

@@ -98,6 +98,7 @@ struct Plan {
     std::vector<int> bucket_nodes;
     std::vector<uint8_t> bucket_clean;    // no exceeded bucket in the 3x3x3 neighbourhood
     bool any_clean = false;
+    bool all_clean = false;               // of the boxes that hold grid nodes: no node takes the template path
     int max_candidates = 0;               // largest candidate count of a clean neighbourhood
     long long informed = 0;               // informed nodes of the mask
 
