@@ -69,7 +69,7 @@ __device__ __forceinline__ void cok_build(const DevJob &J, const DevPlan &P, dou
             // primary_cov(x_r, center); cross_cov(center, x_r) = coef C_x(center - x_r)
             bv[t] = cov_lin(P, qx, qy, qz, o.y, J.err);
             double cx = 0.0;
-            if (cov_in_range(P, qx, qy, qz)) cx = __ldg(J.cross_table + (P.center + o.y));
+            if (cov_in_range(P, qx, qy, qz)) cx = __ldg(J.cross_table + abs(o.y));
             cr[t] = __dmul_rn(J.cok_coef, cx);
         }
         own[t] = o;
@@ -93,7 +93,7 @@ __device__ __forceinline__ void cok_build(const DevJob &J, const DevPlan &P, dou
             if (i < n && k < n && (d < T::NN / 2 || i < T::NN / 2)) {
                 const int2 q = nb[k];
                 const bool in = P.pk.in_range((int)((unsigned)own[t].x - (unsigned)q.x));
-                if (in) v[e] = __ldg(P.table + P.center + abs(own[t].y - q.y));
+                if (in) v[e] = __ldg(P.table + abs(own[t].y - q.y));
                 out |= !in;
             }
         }
@@ -115,7 +115,7 @@ __device__ __forceinline__ void cok_build(const DevJob &J, const DevPlan &P, dou
     for (int e = l; e < T::NR * (T::NC - T::NN); e += T::L) S[T::at(e % T::NR, T::NN + e / T::NR)] = 0.0;
     for (int e = l; e < (T::NR - T::NN) * T::NN; e += T::L) S[T::at(T::NN + e / T::NN, e % T::NN)] = 0.0;
     __syncwarp();
-    const double c0 = __ldg(P.table + P.center);
+    const double c0 = __ldg(P.table);
     for (int i = l; i < T::NR; i += T::L) S[T::at(i, i)] = i < n ? c0 : i == n ? J.cok_svar : 1.0;
 #pragma unroll
     for (int t = 0; t < T::XN; ++t) {
@@ -126,7 +126,7 @@ __device__ __forceinline__ void cok_build(const DevJob &J, const DevPlan &P, dou
             S[T::at(row, T::BCOL)] = bv[t];
         }
     }
-    if (l == 0) S[T::at(n, T::BCOL)] = __dmul_rn(J.cok_coef, __ldg(J.cross_table + P.center));
+    if (l == 0) S[T::at(n, T::BCOL)] = __dmul_rn(J.cok_coef, __ldg(J.cross_table));
     __syncwarp();
 }
 

@@ -145,7 +145,7 @@ __device__ void cok_node(const DevJob &J, const DevPlan &P, CokSmem &S, int node
                 }
             }
         }
-        const double c0 = __ldg(P.table + P.center);
+        const double c0 = __ldg(P.table);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int r = lane + 32 * h;
@@ -154,7 +154,7 @@ __device__ void cok_node(const DevJob &J, const DevPlan &P, CokSmem &S, int node
                 S.A[r * LD + r] = c0;
                 // cross_cov(center, x_r) = coef * C_x(center - x_r); C_x(-v) = C_x(v)
                 double cx = 0.0;
-                if (cov_in_range(P, a.x, a.y, a.z)) cx = __ldg(J.cross_table + (P.center + a.w));
+                if (cov_in_range(P, a.x, a.y, a.z)) cx = __ldg(J.cross_table + abs(a.w));
                 else if (!P.truncated) atomicOr(J.err, DERR_TABLE_RANGE);
                 const double x = __dmul_rn(J.cok_coef, cx);
                 S.A[n * LD + r] = x;
@@ -163,7 +163,7 @@ __device__ void cok_node(const DevJob &J, const DevPlan &P, CokSmem &S, int node
             }
         }
         if (lane == 0) {
-            S.B[n] = __dmul_rn(J.cok_coef, __ldg(J.cross_table + P.center));
+            S.B[n] = __dmul_rn(J.cok_coef, __ldg(J.cross_table));
             S.A[n * LD + n] = J.cok_svar;
         }
         __syncwarp();

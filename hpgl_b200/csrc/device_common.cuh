@@ -23,13 +23,14 @@ __device__ __forceinline__ bool cov_in_range(const DevPlan &P, int vx, int vy, i
            (unsigned)(vz + P.Tz) <= (unsigned)(2 * P.Tz);
 }
 
-// lin = vz*syx + vy*sx + vx, the table offset of v relative to its centre.
+// lin = vz*syx + vy*sx + vx, the table offset of v; C(v) = C(-v) bit for bit, and
+// the table holds the offsets of lin >= 0.
 __device__ __forceinline__ double cov_lin(const DevPlan &P, int vx, int vy, int vz, int lin, int *err) {
     if (!cov_in_range(P, vx, vy, vz)) {
         if (!P.truncated) atomicOr(err, DERR_TABLE_RANGE);
         return 0.0;
     }
-    return __ldg(P.table + (P.center + lin));
+    return __ldg(P.table + abs(lin));
 }
 
 __device__ __forceinline__ double cov_at(const DevPlan &P, int vx, int vy, int vz, int *err) {

@@ -90,6 +90,10 @@ struct Group {
     size_t o_tmpl, o_table, o_bstart, o_bnodes, o_bclean, o_bits;
 };
 
+// The device holds a covariance table (an odd number of entries, symmetric about
+// the middle one, bit for bit) from the middle on: half to copy, half to cache.
+static size_t upper_half(size_t entries) { return entries - entries / 2; }
+
 struct Arena {
     size_t o_values, o_codes, o_mask, o_mean, o_out_values, o_out_codes, o_out_mask, o_probs, o_pk, o_status,
         o_variance, o_weights, o_nb, o_nbcount, o_untouched, o_counters, o_skey, o_sidx, o_svalues,
@@ -311,7 +315,7 @@ static void prepare(JobState &S, const hpgl_b200_job_t &job, const hpgl_b200_res
     A.o_weights = S.want_weights ? take(slots * (S.nmax_all + (S.cok ? 1 : 0)) * 8) : 0;
     A.o_svalues = S.cok ? take(n * 4) : 0;
     A.o_smask = S.cok ? take(n) : 0;
-    A.o_cross = S.cross_table.empty() ? 0 : take(S.cross_table.size() * 8);
+    A.o_cross = S.cross_table.empty() ? 0 : take(upper_half(S.cross_table.size()) * 8);
     A.o_nb = take(n * (size_t)S.nmax_all * 4);
     A.o_nbcount = take(n * 4);
     A.o_untouched = take(n * 4);
@@ -329,7 +333,7 @@ static void prepare(JobState &S, const hpgl_b200_job_t &job, const hpgl_b200_res
                 g.tmpl_dev[i] = make_int4(P.px + P.tmpl[i].dx, P.tmpl[i].dy, P.tmpl[i].dz, P.tmpl[i].delta);
         }, 32768);
         g.o_tmpl = take(g.tmpl_dev.size() * sizeof(int4));
-        g.o_table = take(P.table.size() * 8);
+        g.o_table = take(upper_half(P.table.size()) * 8);
         g.o_bstart = take(P.bucket_start.size() * 4);
         g.o_bnodes = take(P.bucket_nodes.size() * 4);
         g.o_bclean = take(P.bucket_clean.size());
@@ -398,16 +402,16 @@ static void upload_rest(JobState &S, cudaStream_t s) {
         CUDA_CHECK(cudaMemcpyAsync(at<float>(S, A.o_svalues), job.secondary_values, n * 4, cudaMemcpyHostToDevice, s));
         CUDA_CHECK(cudaMemcpyAsync(at<uint8_t>(S, A.o_smask), job.secondary_mask, n, cudaMemcpyHostToDevice, s));
         if (!S.cross_table.empty())
-            CUDA_CHECK(cudaMemcpyAsync(at<double>(S, A.o_cross), S.cross_table.data(), S.cross_table.size() * 8,
-                                       cudaMemcpyHostToDevice, s));
+            CUDA_CHECK(cudaMemcpyAsync(at<double>(S, A.o_cross), S.cross_table.data() + S.cross_table.size() / 2,
+                                       upper_half(S.cross_table.size()) * 8, cudaMemcpyHostToDevice, s));
     }
     for (auto &g : S.groups) {
         const Plan &P = g.plan;
         if (!g.tmpl_dev.empty())
             CUDA_CHECK(cudaMemcpyAsync(at<int4>(S, g.o_tmpl), g.tmpl_dev.data(), g.tmpl_dev.size() * sizeof(int4),
                                        cudaMemcpyHostToDevice, s));
-        CUDA_CHECK(cudaMemcpyAsync(at<double>(S, g.o_table), P.table.data(), P.table.size() * 8,
-                                   cudaMemcpyHostToDevice, s));
+        CUDA_CHECK(cudaMemcpyAsync(at<double>(S, g.o_table), P.table.data() + P.table.size() / 2,
+                                   upper_half(P.table.size()) * 8, cudaMemcpyHostToDevice, s));
         CUDA_CHECK(cudaMemcpyAsync(at<int>(S, g.o_bstart), P.bucket_start.data(), P.bucket_start.size() * 4,
                                    cudaMemcpyHostToDevice, s));
         if (!P.bucket_nodes.empty())
@@ -431,7 +435,6 @@ static void upload_rest(JobState &S, cudaStream_t s) {
         d.Tz = std::min(P.trunc[2], P.B[2]);
         d.sx = 2 * P.B[0] + 1;
         d.syx = d.sx * (2 * P.B[1] + 1);
-        d.center = P.B[2] * d.syx + P.B[1] * d.sx + P.B[0];
         d.truncated = P.truncated ? 1 : 0;
         {
             // offsets reach the radii (template) or 2 r - 1 (clusterizer boxes)

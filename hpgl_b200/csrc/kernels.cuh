@@ -23,12 +23,11 @@ struct DevPlan {
     const int4 *tmpl;        // (packed window offset, dy, dz, node delta)
     int tmpl_len;
     int px, nseg, wpr;
-    // covariance table
+    // covariance table, from offset 0 on: C(v) = table[|vz syx + vy sx + vx|]
     const double *table;
     int Bx, By, Bz;
     int Tx, Ty, Tz;          // half extents read from the table (beyond: 0)
     int sx, syx;             // table strides (x, then y*x)
-    int center;              // table index of offset 0
     int truncated;           // beyond T is the model's 0 (else a broken invariant)
     double c0;
     OffsetPack pk;           // packed neighbour offsets and the range test on their differences

@@ -271,7 +271,7 @@ __device__ int exact64_core(const DevJob &J, const DevPlan &P, Exact64Smem &S, c
     double *U = S.U;
     build_packed<CORR>(J, P, U, S.nb, cs, n, lane, sg);
     const int k0 = lane, k1 = lane + 32;  // the lane's columns in the factorisation
-    const double a_diag = __ldg(P.table + P.center);  // A(k,k) = C(0), the table's centre
+    const double a_diag = __ldg(P.table);  // A(k,k) = C(0)
     // diagonal slots and pads of the lane's columns are zero until their step
 #pragma unroll
     for (int h = 0; h < 2; ++h) {

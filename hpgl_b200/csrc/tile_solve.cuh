@@ -78,8 +78,8 @@ __device__ __forceinline__ void sqrt_rcp(double a, double &root, double &rcp) {
 }
 
 // Entries A(i, k) = C(x_i - x_k) (my_kriging_weights.h:49-58; the tables are
-// exactly symmetric, C(v) = C(-v) bit for bit, so either orientation, and the
-// table's upper half alone, gives the reference's value) of the lane's rows
+// exactly symmetric, C(v) = C(-v) bit for bit, so either orientation gives the
+// reference's value) of the lane's rows
 // of block p at its columns from block p on; the identity beyond n.
 template <typename T>
 __device__ __forceinline__ void tile_gather(const DevJob &J, const DevPlan &P, const int2 *nb, int n, int r,
@@ -96,7 +96,7 @@ __device__ __forceinline__ void tile_gather(const DevJob &J, const DevPlan &P, c
             const int2 q = nb[k];
             const bool live = i < n && k < n, in = P.pk.in_range((int)((unsigned)o.x - (unsigned)q.x));
             a[h][b] = i == k ? 1.0 : 0.0;
-            if (live && in) a[h][b] = __ldg(P.table + P.center + abs(o.y - q.y));
+            if (live && in) a[h][b] = __ldg(P.table + abs(o.y - q.y));
             out |= live && !in;
         }
     }
