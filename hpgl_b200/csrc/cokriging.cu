@@ -337,9 +337,9 @@ static void launch_cok_tile(const DevJob &J, const DevPlan &P, cudaStream_t s) {
 // 0.88 M systems (161x119x47) in ms, in brackets one system a warp with a row
 // per lane in shared memory:
 //   8: 0.44 [4.5]   12: 0.82 [6.5]   16: 1.76 [8.8]   20: 3.06 [11.2]
-//   24: 4.52 [13.7]   28: 6.65 [16.5]   36: 11.5 [26.4]   40: 17.0 [32.3]
+//   24: 4.46 [13.7]   28: 6.65 [16.5]   36: 11.5 [26.4]   40: 17.0 [32.3]
 //   44: 19.7 [38.5]   48: 28.8 [52.6]
-// and of 4.11 M (256x256x64): 32: 38.1 [90.9].  Neighbouring tiles: 12 as 8
+// and of 4.11 M (256x256x64): 32: 37.5 [90.9].  Neighbouring tiles: 12 as 8
 // lanes 1.09, 16 as 16 lanes 2.29, 24 as 16 lanes 4.61, 32 as a whole warp
 // 47.8, 36 as a whole warp 13.6.  Above 48 the square no longer fits a warp's
 // registers.

@@ -155,7 +155,7 @@ void launch_search_cluster(const DevJob &J, const DevPlan &P, double *scratch_ke
                            int n_warps, cudaStream_t s);
 // Every node's system (the tiled FP64 solves, for either precision: an FP32
 // inverse with FP64 refinement, which mixed requests once ran, took 22.5 ms
-// where they take 17.9 at 32 neighbours and 0.82 of the one-system-a-warp
+// where they take 17.5 at 32 neighbours and 0.82 of the one-system-a-warp
 // solve, about twice theirs, above).
 void launch_solve(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm = 0);
 void launch_ik_argmax(const DevJob &J, cudaStream_t s);

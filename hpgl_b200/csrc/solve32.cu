@@ -730,9 +730,9 @@ void launch_fused32(const DevJob &J, const DevPlan &P, cudaStream_t s, int block
 // the panel (row blocks whose sums are kept open together) is the widest
 // that does not spill.  Solve of the IK 200x200x100 job (4.0 M systems) with
 // the neighbour count set, in ms:
-//   8: 1.09   12: 2.03   16: 3.11   20: 7.1   24: 9.2   28: 14.7
+//   8: 1.06   12: 1.99   16: 3.09   20: 7.1   24: 9.1   28: 14.5
 // against 39.7 at 24 with one column per lane and one system a warp; SK
-// 256x256x64 (4.15 M systems, 32 neighbours) 17.9 against 53.2, OK 20.2
+// 256x256x64 (4.15 M systems, 32 neighbours) 17.5 against 53.2, OK 19.7
 // against 57.1.  The neighbouring tiles, measured on earlier builds: 12 as 8
 // lanes 3.5; 16 as 8 lanes 5.2; 20 as 8 lanes 8.4; 24 as 8 lanes 9.6; 32 as
 // 16 lanes 21.0 where 8 lanes took 19.2.

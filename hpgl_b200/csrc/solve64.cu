@@ -668,9 +668,9 @@ __global__ void __launch_bounds__(WARPS64_BLOCK * 32) k_sis_try64(DevJob J, cons
 // than the better occupancy gives: issue slots in use 48 % for 31 %.  At 56
 // and below they cost more (56: 85.2, 48: 61.0, 40: 43.8 ms).  Solve of SK
 // 256x256x64 (4.15 M systems) with the neighbour count set, in ms (one system
-// a warp, two columns a lane): 36: 28.3   40: 33.2 [149.6]   44: 39.8   48:
-// 46.8 [181.7]   52: 68.0   56: 77.1 [211.3]   64: 107.1 [241.7], 123.2 with
-// 16 lanes; LVM 512x512x32 (7.5 M systems, 64) 182.7 [327], with 16
+// a warp, two columns a lane): 36: 28.8   40: 34.0 [149.6]   44: 40.7   48:
+// 45.1 [181.7]   52: 66.2   56: 76.3 [211.3]   64: 106.1 [241.7], 123.2 with
+// 16 lanes; LVM 512x512x32 (7.5 M systems, 64) 175.7 [327], with 16
 // lanes 244.
 void launch_solve64(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
     const int b = blocks_per_sm;

@@ -3,7 +3,7 @@
 // several systems per warp, each spread over a two-dimensional cyclic tile of
 // lanes.
 //
-// Measured on SK 256x256x64 (4.15 M systems of 32 neighbours): 17.9 ms where
+// Measured on SK 256x256x64 (4.15 M systems of 32 neighbours): 17.5 ms where
 // one column per lane and one system a warp took 53.2 ms.  ncu on the
 // 128x128x32 cube: 2 300 instructions a system (8 387), FP64 pipe 30 %, the
 // shared-memory / L1 data pipe 58 %, 8 warps an SM (their registers hold the
