@@ -283,8 +283,11 @@ static void launch_block(double *out, const float *center, const float *xs, cons
     }
     for (int i = 0; i < 3; ++i) a.xyz[3 * n + i] = center[i];
     const size_t smem = weights_smem(n);
+    // The limit is the kernel's, not the launch's, and the two entries do not
+    // exclude each other: every call sets it to the same value.
     if (smem > 48 * 1024)
-        WCHECK(cudaFuncSetAttribute(k_sk_weights_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        WCHECK(cudaFuncSetAttribute(k_sk_weights_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)weights_smem(BLOCK_MAX)));
     k_sk_weights_block<<<1, BLOCK_THREADS, smem, s>>>(a, out);
     WCHECK(cudaGetLastError());
 }
