@@ -602,8 +602,11 @@ struct DevMem {
         p.push_back(q);
         return static_cast<T *>(q);
     }
+    // Waits for the stream, on every way out of the call: the caller's arrays
+    // may be pinned, and a copy of one must not outlive the call.
     ~DevMem() {
         for (void *q : p) cudaFreeAsync(q, s);
+        cudaStreamSynchronize(s);
     }
 };
 
@@ -703,13 +706,6 @@ void cv_grid(const variogram_search_template_t &t, const hard_data_t &hd, int re
     const long long ncell_all = (long long)hd.m_data_shape[0] * hd.m_data_shape[1] * hd.m_data_shape[2];
     if (nwin <= 0 || ncell_all <= 0) return;
     const CvT T = cv_t(t, lags);
-    // the walked cells must lie in the mask too (the reference reads both at
-    // the same coordinates)
-    auto shapes = [&] {
-        for (int i = 0; i < 3; ++i)
-            if (hd.m_data_shape[i] > hd.m_mask_shape[i])
-                throw HpglError{HPGL_E_INVALID, "the mask is smaller than the data"};
-    };
     // offsets in the tunnel with a non-empty lag range, in the walk's order
     int2 *d_range = M.alloc<int2>((size_t)nwin);
     k_cv_offsets<<<(unsigned)((nwin + NT - 1) / NT), NT, 0, s>>>(T, i0, j0, k0, nj, nk, nwin, d_range);
@@ -729,16 +725,20 @@ void cv_grid(const variogram_search_template_t &t, const hard_data_t &hd, int re
         reach = std::max(reach, std::abs(i0 + a));
     }
     if (!any) return;
-    // data and mask on the device
     const long long dspan = span(hd.m_data_shape, hd.m_data_strides), mspan = span(hd.m_mask_shape, hd.m_mask_strides);
+    // the walked cells must lie in the mask too (the reference reads both at
+    // the same coordinates)
+    for (int i = 0; i < 3; ++i)
+        if (hd.m_data_shape[i] > hd.m_mask_shape[i])
+            throw HpglError{HPGL_E_INVALID, "the mask is smaller than the data"};
+    if (offs.empty()) return;
+    // data and mask on the device
     float *d_data = M.alloc<float>((size_t)dspan);
     unsigned char *d_mask = M.alloc<unsigned char>((size_t)mspan);
     CV_CHECK(cudaMemcpyAsync(d_mask, hd.m_mask, (size_t)mspan, cudaMemcpyHostToDevice, s));
-    shapes();
     Grid G{d_data, d_mask, hd.m_data_shape[0], hd.m_data_shape[1], hd.m_data_shape[2], hd.m_mask_shape[0],
            hd.m_mask_shape[1], hd.m_mask_shape[2], hd.m_data_strides[0], hd.m_data_strides[1],
            hd.m_data_strides[2], hd.m_mask_strides[0], hd.m_mask_strides[1], hd.m_mask_strides[2]};
-    if (offs.empty()) return;
     // informed cells: bit rows of the mask, and the walked words with any
     const int wxm = (G.mx + 31) / 32, wx = (G.nx + 31) / 32, pad = (reach + 31) / 32;
     const int wpr = wxm + 2 * pad + 1;
