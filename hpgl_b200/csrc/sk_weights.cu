@@ -300,14 +300,21 @@ static void take_weights(const double *x, int n, float *weights) {
 
 static std::mutex g_weights_mutex;
 
-// Where the block kernel leaves its result: 1.3 kB of pinned host memory that
-// the device writes to directly, kept for the process, used under
-// g_weights_mutex.
-static double *weights_mailbox() {
-    static double *box = nullptr;
-    if (!box)
-        WCHECK(cudaHostAlloc(&box, (BLOCK_MAX + 1) * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped));
-    return box;
+// Where the block kernel leaves its result: a page of the library's own memory
+// that the device writes to directly, used under g_weights_mutex.  It is
+// registered on the first call, and again when a reset of the device has
+// dropped the registration; as the page is never anyone else's, an address that
+// the device knows is always this one.
+alignas(4096) static unsigned char g_mailbox[4096];
+static_assert((BLOCK_MAX + 1) * sizeof(double) <= sizeof(g_mailbox), "room for the weights and the status");
+
+static double *mailbox_on_device() {
+    double *out = nullptr;
+    if (cudaHostGetDevicePointer(&out, g_mailbox, 0) == cudaSuccess) return out;
+    cudaGetLastError();
+    WCHECK(cudaHostRegister(g_mailbox, sizeof(g_mailbox), cudaHostRegisterPortable | cudaHostRegisterMapped));
+    WCHECK(cudaHostGetDevicePointer(&out, g_mailbox, 0));
+    return out;
 }
 
 void sk_weights_alloc(const float *center, const float *xs, const float *ys, const float *zs, int n,
@@ -319,11 +326,9 @@ void sk_weights_alloc(const float *center, const float *xs, const float *ys, con
     if (n == 0) return;
     std::lock_guard<std::mutex> lock(g_weights_mutex);
     if (n <= BLOCK_MAX) {
-        double *box = weights_mailbox(), *out = nullptr;
-        WCHECK(cudaHostGetDevicePointer(&out, box, 0));
-        launch_block(out, center, xs, ys, zs, n, cov, cudaStreamPerThread);
+        launch_block(mailbox_on_device(), center, xs, ys, zs, n, cov, cudaStreamPerThread);
         WCHECK(cudaStreamSynchronize(cudaStreamPerThread));
-        take_weights(box, n, weights);
+        take_weights(reinterpret_cast<const double *>(g_mailbox), n, weights);
         return;
     }
     double *scratch = nullptr;
