@@ -909,26 +909,28 @@ static void sgs_run(JobState &S, hpgl_b200_result_t &res, SyncContext &C, std::c
     const size_t o_ctl = take(sizeof(SgsCtl)), o_nodes = take((size_t)nsim * 4), o_xp = take((size_t)nsim * 8),
                  o_rank = take((size_t)S.size * 4), o_pend = take(bits_bytes), o_blocker = take((size_t)nsim * 4),
                  o_done = take((size_t)nsim), o_w0 = take((size_t)window * 4), o_w1 = take((size_t)window * 4),
-                 o_ok = take((size_t)window), o_try = take((size_t)window * 4),
-                 o_solve = take((size_t)window * 4);
-    // Indicator simulation: the category groups with their own search and
-    // system (two categories krige category 0 only), solved apart by the tiled
-    // kernels unless the correlogram weights scale every category's system
-    // differently, a group is not theirs, or the lists by window slot would
-    // pass 1 GiB.
+                 o_ok = take((size_t)window), o_try = take((size_t)window * 4);
+    // Where the systems are solved apart by the tiled kernels the neighbour
+    // lists lie by window slot, one per group of categories with its own search
+    // and system (indicator simulation; two categories krige category 0 only),
+    // unless the correlogram weights scale every category's system differently,
+    // a plan is not the tiles', or the lists would pass 1 GiB.  No slot beyond the
+    // nodes to simulate is ever used.
+    const size_t slots = (size_t)std::max<long long>(1, std::min<long long>(window, nsim));
     std::vector<SisGroup> sis_groups;
-    if (indicator && !S.job.correlogram) {
+    if (indicator && !S.job.correlogram)
         for (auto &gr : S.groups) {
             if (S.K == 2 && gr.k0 > 0) continue;
             sis_groups.push_back(SisGroup{gr.dp, gr.k0, S.K == 2 ? 1 : gr.k1});
         }
-        bool tiles = sis_groups.size() * (size_t)window * (size_t)S.nmax_all * 4 <= (size_t)1 << 30;
-        for (auto &q : sis_groups) tiles = tiles && sis_tiles(q.plan);
-        if (!tiles) sis_groups.clear();
-    }
-    const size_t lists = std::max<size_t>(1, sis_groups.size());
-    const size_t o_lists = take(lists * (size_t)window * (size_t)S.nmax_all * 4),
-                 o_counts = take(lists * (size_t)window * 4);
+    const size_t lists = indicator ? sis_groups.size() : 1;
+    bool tiles = lists > 0 && lists * slots * (size_t)S.nmax_all * 4 <= (size_t)1 << 30;
+    if (!indicator) tiles = tiles && sim_tiles(g.dp);
+    for (auto &q : sis_groups) tiles = tiles && sim_tiles(q.plan);
+    if (!tiles) sis_groups.clear();
+    const size_t o_solve = take(tiles ? slots * 4 : 0),
+                 o_lists = take(tiles ? lists * slots * (size_t)S.nmax_all * 4 : 0),
+                 o_counts = take(tiles ? lists * slots * 4 : 0);
     std::vector<DevPlan> cat_plans;  // indicator simulation: every category's plan (its group's)
     if (indicator)
         for (auto &gr : S.groups)
@@ -951,9 +953,12 @@ static void sgs_run(JobState &S, hpgl_b200_result_t &res, SyncContext &C, std::c
     G.win1 = reinterpret_cast<int *>(scratch + o_w1);
     G.ok = scratch + o_ok;
     G.trylist = reinterpret_cast<int *>(scratch + o_try);
-    G.solvelist = reinterpret_cast<int *>(scratch + o_solve);
-    G.lists = reinterpret_cast<int *>(scratch + o_lists);
-    G.counts = reinterpret_cast<int *>(scratch + o_counts);
+    G.solvelist = G.lists = G.counts = nullptr;
+    if (tiles) {
+        G.solvelist = reinterpret_cast<int *>(scratch + o_solve);
+        G.lists = reinterpret_cast<int *>(scratch + o_lists);
+        G.counts = reinterpret_cast<int *>(scratch + o_counts);
+    }
     DevPlan *d_plans = reinterpret_cast<DevPlan *>(scratch + o_plans);
     SisGroups sis;
     if (!sis_groups.empty()) {

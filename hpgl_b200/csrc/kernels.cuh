@@ -195,7 +195,8 @@ struct SgsState {
     int *win0, *win1;       // window buffers (path ranks)
     uint8_t *ok;            // per window slot: the node committed this round
     int *trylist;           // window slots tried this round (blocker committed or none)
-    int *solvelist;         // of those, the slots whose search completed
+    // where the tiled kernels solve the systems (sim_tiles), else null:
+    int *solvelist;         // of the slots tried, those whose search completed
     int *lists, *counts;    // per window slot (and category group): its neighbours and their number
 };
 // rank_of from the mask and the path
@@ -222,8 +223,8 @@ struct SisGroups {
     const DevPlan *dev = nullptr;
     int n = 0, stride = 0;
 };
-// whether the tiled kernels take a plan's systems (tile_solve.cuh)
-bool sis_tiles(const DevPlan &P);
+// whether the tiled kernels take a plan's systems in simulation (tile_solve.cuh)
+bool sim_tiles(const DevPlan &P);
 void launch_sis_round(const DevJob &J, const DevPlan &P0, const DevPlan *plans, int family, const SisGroups &groups,
                       const SgsState &G, int cur, cudaStream_t s);
 void launch_sis_groups(const DevJob &J, const SisGroups &groups, const SgsState &G, int cur, cudaStream_t s);

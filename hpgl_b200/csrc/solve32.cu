@@ -669,7 +669,7 @@ __global__ void __launch_bounds__(256) k_sis_draw(DevJob J, SgsState G, int cur)
     }
 }
 
-bool sis_tiles(const DevPlan &P) { return P.nmax <= 32 && tile_takes(P); }
+bool sim_tiles(const DevPlan &P) { return P.nmax <= 32 && tile_takes(P); }
 
 void launch_sis_groups(const DevJob &J, const SisGroups &groups, const SgsState &G, int cur, cudaStream_t s) {
     const long long g = persistent_grid((const void *)k_sis_search, 256, 0, 0, 1LL << 30);
@@ -689,7 +689,7 @@ void launch_sis_groups(const DevJob &J, const SisGroups &groups, const SgsState 
 }
 
 void launch_sgs_try32(const DevJob &J, const DevPlan &P, const SgsState &G, int cur, cudaStream_t s) {
-    if (tile_takes(P)) {
+    if (G.lists) {
         const long long g = persistent_grid((const void *)k_sgs_search, 256, 0, 0, 1LL << 30);
         k_sgs_search<<<(unsigned)g, 256, 0, s>>>(J, P, G, cur);
         if (P.nmax <= 8) launch_sgs_solve<TileGeom<8, 4, 1, 2, 10>, 4, 5>(J, P, G, cur, s);
