@@ -582,6 +582,10 @@ int hpgl_b200_variogram_stats(variogram_search_template_t *templ, hard_data_t *d
     });
 }
 
+int hpgl_b200_variogram_release(void) {
+    return guarded("hpgl_b200_variogram_release", [] { cv_release(); });
+}
+
 // Sequential Gaussian simulation (api.cpp:409-469 of the reference), in
 // place on the property.  With a CDF the informed values (and the LVM mean
 // cube) are normal-score transformed first and every informed value is

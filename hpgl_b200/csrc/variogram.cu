@@ -573,11 +573,12 @@ cudaStream_t cv_stream() {
 // Device memory of a call, from a pool of this file's own: freed in stream
 // order at scope exit, and up to POOL_KEEP bytes of what was freed stay with
 // the pool for the next call (a cudaMalloc and cudaFree of each buffer per
-// call took between 1 and 30 ms); more goes back to the device.
+// call took between 1 and 30 ms); more goes back to the device
+// (cv_release gives that back as well).
 constexpr unsigned long long POOL_KEEP = 256ull << 20;
+cudaMemPool_t g_pool = nullptr;  // guarded by g_cv_mutex
 cudaMemPool_t cv_pool() {
-    static cudaMemPool_t pool = nullptr;
-    if (!pool) {
+    if (!g_pool) {
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -586,9 +587,9 @@ cudaMemPool_t cv_pool() {
         CV_CHECK(cudaMemPoolCreate(&q, &props));
         unsigned long long keep = POOL_KEEP;
         CV_CHECK(cudaMemPoolSetAttribute(q, cudaMemPoolAttrReleaseThreshold, &keep));
-        pool = q;
+        g_pool = q;
     }
-    return pool;
+    return g_pool;
 }
 
 struct DevMem {
@@ -656,6 +657,11 @@ void window_of(const variogram_search_template_t &t, double w[6]) {
 }
 
 }  // namespace
+
+void cv_release() {
+    std::lock_guard<std::mutex> lock(g_cv_mutex);
+    if (g_pool) CV_CHECK(cudaMemPoolTrimTo(g_pool, 0));
+}
 
 void cv_fill_ellipsoid(ellipsoid_t *ell, double azimuth, double dip, double rotation) {
     // ellipsoid.cpp:40-72: M = (A B) C with the reference's value of pi

@@ -20,4 +20,7 @@ void cv_points(const variogram_search_template_t &t, const cont_point_set_t &poi
 void cv_stack_layers(const float_data_t *layers, const int *markers, int nlayers, int nz, float scalez, int blank,
                      float_data_t *result);
 
+// Gives the device memory kept between calls back.
+void cv_release();
+
 }  // namespace hpgl_b200

@@ -11,7 +11,8 @@ Differences from the reference:
   "Z" and "Property" arrays (the reference's version calls the dict and uses
   an undefined name, so it never ran);
 * every call checks the library's last-error state and raises HpglError;
-* ``CalcVariogramStats`` returns the per-lag pair counts and sums as well.
+* ``CalcVariogramStats`` returns the per-lag pair counts and sums as well;
+* ``ReleaseMemory`` gives back the device memory kept between calls.
 """
 
 import ctypes as C
@@ -23,7 +24,7 @@ from .geo_bsd.hpgl_wrap import _hpgl_so as cvar
 from .geo_bsd.hpgl_wrap import HpglError, check_last_error
 
 __all__ = ["Ellipsoid", "VariogramSearchTemplate", "CalcVariograms", "CalcVariogramsFromPointSet",
-           "CalcVariogramStats", "CStackLayers", "HpglError"]
+           "CalcVariogramStats", "CStackLayers", "ReleaseMemory", "HpglError"]
 
 
 class vector_t(C.Structure):
@@ -69,6 +70,9 @@ cvar.hpgl_b200_variogram_stats.restype = C.c_int
 cvar.hpgl_b200_variogram_stats.argtypes = [C.POINTER(variogram_search_template_t), C.POINTER(hard_data_t),
                                            C.POINTER(cont_point_set_t), C.c_int, C.c_int,
                                            NC.ndpointer(dtype=numpy.float64), NC.ndpointer(dtype=numpy.int64)]
+
+cvar.hpgl_b200_variogram_release.restype = C.c_int
+cvar.hpgl_b200_variogram_release.argtypes = []
 
 
 def _strides(array):
@@ -178,3 +182,9 @@ def CStackLayers(layers, markers, nz, scalez, blank_value, result):
                            len(layers2), nz, scalez, blank_value, C.byref(_float_data(result)))
     check_last_error()
     return result
+
+
+def ReleaseMemory():
+    """Gives the device memory that the calls keep for the next one back."""
+    cvar.hpgl_b200_variogram_release()
+    check_last_error()

@@ -93,6 +93,11 @@ int hpgl_b200_variogram_stats(struct variogram_search_template_t *templ, struct 
                               struct cont_point_set_t *points, int result_length, int percentToUse,
                               double *sums, long long *counts);
 
+/* The functions above keep up to 256 MB of freed device memory for the next
+   call.  Gives it back to the device; the next call takes its memory anew.
+   Returns 0 or an HPGL_E_* code. */
+int hpgl_b200_variogram_release(void);
+
 #ifdef __cplusplus
 }
 #endif
