@@ -700,6 +700,7 @@ static void download(const JobState &S, hpgl_b200_result_t &res, const Counters 
 struct SyncContext {
     cudaStream_t stream = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;  // around a job's device pass
+    cudaEvent_t staged = nullptr;            // its outputs are in the staging
     char *arena = nullptr;
     size_t cap = 0;
     char *inputs = nullptr;   // the job's inputs, uploaded while it is planned
@@ -720,8 +721,7 @@ static SyncContext &sync_ctx() {
         ensure_device();
         auto *nc = new SyncContext();
         CUDA_CHECK(cudaStreamCreateWithFlags(&nc->stream, cudaStreamNonBlocking));
-        CUDA_CHECK(cudaEventCreate(&nc->e0));
-        CUDA_CHECK(cudaEventCreate(&nc->e1));
+        for (cudaEvent_t *e : {&nc->e0, &nc->e1, &nc->staged}) CUDA_CHECK(cudaEventCreate(e));
         c = nc;
     }
     return *c;
@@ -803,6 +803,7 @@ void run_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res) {
     std::lock_guard<std::mutex> lock(g_sync_mutex);
     SyncContext &C = sync_ctx();
     char *staging = nullptr;
+    std::chrono::steady_clock::time_point t1;  // planned
     if (early_inputs(job)) {
         // The inputs go to pinned staging and on to the device on a helper
         // thread while this one plans the job; the same layout function
@@ -840,16 +841,15 @@ void run_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res) {
             std::rethrow_exception(copy_error);
         }
         if (S.ar.in_total != in_total) throw HpglError{HPGL_E_INTERNAL, "input layout changed while planning"};
-        auto t1 = std::chrono::steady_clock::now();
+        t1 = std::chrono::steady_clock::now();
         sync_arena(C, S.ar.total - in_total);
         S.in_base = C.inputs;
         S.rest = C.arena;
         // The pass follows on the same stream, with no wait for the uploads:
         // a copy from pageable memory returns once its source has been read.
         upload_rest(S, C.stream);
-        res.ms_h2d = ms_since(t1);
     } else {
-        auto t1 = std::chrono::steady_clock::now();
+        t1 = std::chrono::steady_clock::now();
         sync_arena(C, S.ar.total);
         set_arena(S, C.arena);
         upload(S, C.stream);
@@ -863,14 +863,24 @@ void run_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res) {
     });
     CUDA_CHECK(cudaEventRecord(C.e1, C.stream));
     // one wait for the pass, its counters and its staged outputs
-    if (staging) stage_outputs(S, C.stream, staging);
+    if (staging) {
+        stage_outputs(S, C.stream, staging);
+        CUDA_CHECK(cudaEventRecord(C.staged, C.stream));
+    }
     Counters cnt = read_counters(S, C.stream);
     float ms = 0;
     cudaEventElapsedTime(&ms, C.e0, C.e1);
     res.ms_device = ms;
+    float down = 0;
+    if (staging) {
+        // the one wait covers the rest of the uploads, the pass and the outputs'
+        // copy into the staging
+        cudaEventElapsedTime(&down, C.e1, C.staged);
+        res.ms_h2d = std::max(0.0, ms_since(t1) - ms - down);
+    }
     auto t2 = std::chrono::steady_clock::now();
     download(S, res, cnt, C.stream, staging);
-    res.ms_d2h = ms_since(t2);
+    res.ms_d2h = ms_since(t2) + down;
     res.ms_total = ms_since(t0);
 }
 

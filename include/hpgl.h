@@ -356,9 +356,9 @@ typedef struct hpgl_b200_result_t {
     long long systems_fp64;       /* of those, solved by the FP64 path */
     long long failures;           /* no neighbours + singular */
     double ms_plan;               /* host planning (template, tables, buckets) */
-    double ms_h2d;
+    double ms_h2d;                /* uploads after planning (the inputs' beside it not counted) */
     double ms_device;             /* device work, CUDA events */
-    double ms_d2h;
+    double ms_d2h;                /* outputs to the caller's arrays, by way of staging */
     double ms_total;              /* wall time of the call */
     long long rounds;             /* sequential simulation: speculative rounds */
 } hpgl_b200_result_t;
