@@ -345,7 +345,7 @@ static void launch_cok_tile(const DevJob &J, const DevPlan &P, cudaStream_t s) {
 // registers.
 void launch_cokriging(const DevJob &J, const DevPlan &P, cudaStream_t s) {
     if (J.size <= 0) return;
-    if (P.pk.m == 0 || P.nmax > 48) launch_general(J, P, false, s);
+    if (!cok_tile_takes(P)) launch_general(J, P, false, s);
     else if (P.nmax <= 8) launch_cok_tile<CokGeom<8, 4, 1>, 4, 4>(J, P, s);
     else if (P.nmax <= 12) launch_cok_tile<CokGeom<12, 4, 1>, 4, 3>(J, P, s);
     else if (P.nmax <= 16) launch_cok_tile<CokGeom<16, 4, 2>, 4, 3>(J, P, s);

@@ -1063,9 +1063,14 @@ static void sgs_run(JobState &S, hpgl_b200_result_t &res, SyncContext &C, std::c
     res.rounds = hc.rounds;
 }
 
-static const char *top_kernel_name(int nmax, int schedule) {
-    if (schedule == SCHED_FUSED) return nmax <= 32 ? "k_fused32" : "k_fused64";
-    return "k_solve_tile";
+// The kernel that solves a job's systems, by the rules of the launches.
+static const char *top_kernel_name(const JobState &S) {
+    const DevPlan &P = S.groups[0].dp;
+    if (S.cok) return cok_tile_takes(P) ? "k_cok_tile" : "k_cokriging";
+    if (tuning_get(tuning_family(P.nmax), S.precision).schedule == SCHED_FUSED)
+        return P.nmax <= 32 ? "k_fused32" : "k_fused64";
+    if (tile_takes(P)) return "k_solve_tile";
+    return P.nmax <= 32 ? "k_solve_exact32" : "k_solve_exact64";
 }
 
 // The job's device pass captured once as a CUDA graph and replayed for every
@@ -1149,10 +1154,7 @@ void bench_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res, hpgl_b200_be
     bench.ms_top_kernel = top_sum / phase_runs;
     bench.ms_search = search_sum / phase_runs;
     bench.ms_resolve = resolve_sum / phase_runs;
-    snprintf(bench.top_kernel, sizeof(bench.top_kernel), "%s",
-             S.cok ? (S.groups[0].dp.pk.m != 0 && S.nmax_all <= 48 ? "k_cok_tile" : "k_cokriging")
-                   : top_kernel_name(S.nmax_all,
-                                     tuning_get(tuning_family(S.nmax_all), S.precision).schedule));
+    snprintf(bench.top_kernel, sizeof(bench.top_kernel), "%s", top_kernel_name(S));
     bench.launches_per_iter = pt.launches;
     cudaEventDestroy(pt.search0);
     cudaEventDestroy(pt.top0);

@@ -148,6 +148,15 @@ inline int tuning_family(int nmax) { return nmax <= 32 ? 0 : 1; }
 // grid for a persistent kernel: min(units, SMs x min(blocks_per_sm, occupancy))
 long long persistent_grid(const void *fn, int threads, size_t smem, int blocks_per_sm, long long units);
 
+// The jobs the tiled kernels take: neighbour offsets that pack into one word
+// (OffsetPack: extents and ranges whose fields need at most 32 bits together)
+// and a sill whose pivots stay in sqrt_rcp's range.  The others keep the
+// one-system-a-warp kernels.
+constexpr double PIVOT_C0_MIN = 0x1p-600, PIVOT_C0_MAX = 0x1p+700;
+inline bool tile_takes(const DevPlan &P) { return P.pk.m != 0 && P.c0 >= PIVOT_C0_MIN && P.c0 < PIVOT_C0_MAX; }
+// ... and the tiled cokriging, whose square fits a warp's registers up to 48.
+inline bool cok_tile_takes(const DevPlan &P) { return P.pk.m != 0 && P.nmax <= 48; }
+
 // Launchers (stream-ordered, no synchronisation).
 void launch_build_bits(const DevJob &J, const DevPlan &P, uint32_t *bits, cudaStream_t s);
 void launch_search_template(const DevJob &J, const DevPlan &P, cudaStream_t s);

@@ -60,7 +60,6 @@ struct alignas(16) TileTables {
 // rounding up of the step before excludes.  Equal to __dsqrt_rn and __drcp_rn
 // bit for bit for 2^-767 <= a < 2^769 (tests/test_tile_solve.py); a <= 0 or
 // NaN, a singular system, gives what nobody reads.
-constexpr double PIVOT_C0_MIN = 0x1p-600, PIVOT_C0_MAX = 0x1p+700;
 __device__ __forceinline__ void sqrt_rcp(double a, double &root, double &rcp) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
@@ -674,11 +673,6 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_sgs_solve(DevJob J, DevPla
         __syncwarp();
     }
 }
-
-// The jobs the tiled kernels take: neighbour offsets that pack into one word
-// (extents up to several hundred cells on every axis) and a sill whose pivots
-// stay in sqrt_rcp's range.  The others keep the one-system-a-warp kernels.
-inline bool tile_takes(const DevPlan &P) { return P.pk.m != 0 && P.c0 >= PIVOT_C0_MIN && P.c0 < PIVOT_C0_MAX; }
 
 // The same for indicator simulation: the system of categories [k0, k1), which
 // share a covariance model and search, solved once; per category the
