@@ -192,8 +192,7 @@ __global__ void k_cv_offsets(CvT T, int i0, int j0, int k0, int nj, int nk, long
 struct Grid {
     const float *data;
     const unsigned char *mask;
-    int nx, ny, nz;        // data shape (the cells walked)
-    int mx, my, mz;        // mask shape (the bounds of the paired cell)
+    int nx, ny, nz;        // data shape
     int ds0, ds1, ds2;     // data strides (elements)
     int ms0, ms1, ms2;     // mask strides
 };
@@ -201,15 +200,15 @@ struct Grid {
 // The informed cells of the mask as bit rows: row (y, z) of `wpr` words, the
 // cells of x at bit `pad` words + x, zero words around them, so that a word of
 // cells displaced by any offset of the window is two words and a funnel
-// shift, zero where it leaves the mask.  One warp per word.
+// shift, zero where it leaves the data.  One warp per word.
 __global__ void k_cv_bits(Grid G, int wx, int wpr, int pad, long long nwords, unsigned *bits) {
     const long long i = (blockIdx.x * (long long)NT + threadIdx.x) >> 5;
     if (i >= nwords) return;
-    const int w = (int)(i % wx), y = (int)(i / wx % G.my), z = (int)(i / ((long long)wx * G.my));
+    const int w = (int)(i % wx), y = (int)(i / wx % G.ny), z = (int)(i / ((long long)wx * G.ny));
     const int x = w * 32 + (threadIdx.x & 31);
-    const bool inf = x < G.mx && G.mask[(long long)x * G.ms0 + (long long)y * G.ms1 + (long long)z * G.ms2] != 0;
+    const bool inf = x < G.nx && G.mask[(long long)x * G.ms0 + (long long)y * G.ms1 + (long long)z * G.ms2] != 0;
     const unsigned b = __ballot_sync(FULL_MASK, inf);
-    if ((threadIdx.x & 31) == 0) bits[((long long)z * G.my + y) * wpr + pad + w] = b;
+    if ((threadIdx.x & 31) == 0) bits[((long long)z * G.ny + y) * wpr + pad + w] = b;
 }
 
 // Word i of the walked cells (the data's shape, x fastest).
@@ -219,9 +218,7 @@ __device__ __forceinline__ unsigned walk_word(const Grid &G, const unsigned *bit
     w = (int)(i % wx);
     y = (int)(i / wx % G.ny);
     z = (int)(i / ((long long)wx * G.ny));
-    const unsigned b = bits[((long long)z * G.my + y) * wpr + pad + w];
-    const int left = G.nx - w * 32;
-    return left < 32 ? b & ((1u << left) - 1u) : b;
+    return bits[((long long)z * G.ny + y) * wpr + pad + w];
 }
 
 // words with informed cells per block of NT words; the informed cells of all
@@ -318,9 +315,9 @@ __global__ void __launch_bounds__(NT) k_cv_pairs(Grid G, const unsigned *bits, i
     for (long long c = c0 + threadIdx.x; c < c1; c += NT) {
         const int4 q = words[c];
         const int y = q.y + f.y, z = q.z + f.z;
-        if ((unsigned)y >= (unsigned)G.my || (unsigned)z >= (unsigned)G.mz) continue;
+        if ((unsigned)y >= (unsigned)G.ny || (unsigned)z >= (unsigned)G.nz) continue;
         const int xb = q.x * 32 + from;
-        const unsigned *row = bits + ((long long)z * G.my + y) * wpr + (xb >> 5);
+        const unsigned *row = bits + ((long long)z * G.ny + y) * wpr + (xb >> 5);
         unsigned m = (unsigned)q.w & __funnelshift_r(row[0], row[1], xb & 31);
         if (!m) continue;
         const float *d0 = G.data + (long long)q.x * 32 * G.ds0 + (long long)q.y * G.ds1 + (long long)q.z * G.ds2;
@@ -725,8 +722,8 @@ void cv_grid(const variogram_search_template_t &t, const hard_data_t &hd, int re
         if (range[idx].x < 0) continue;
         any = true;
         const int c = (int)(idx % nk), b = (int)((idx / nk) % nj), a = (int)(idx / ((long long)nk * nj));
-        // an offset as long as the mask pairs nothing
-        if (std::abs(i0 + a) >= hd.m_mask_shape[0]) continue;
+        // an offset as long as the data pairs nothing
+        if (std::abs(i0 + a) >= hd.m_data_shape[0]) continue;
         offs.push_back(Offset{i0 + a, j0 + b, k0 + c, range[idx].x, range[idx].y, idx});
         reach = std::max(reach, std::abs(i0 + a));
     }
@@ -742,16 +739,17 @@ void cv_grid(const variogram_search_template_t &t, const hard_data_t &hd, int re
     float *d_data = M.alloc<float>((size_t)dspan);
     unsigned char *d_mask = M.alloc<unsigned char>((size_t)mspan);
     CV_CHECK(cudaMemcpyAsync(d_mask, hd.m_mask, (size_t)mspan, cudaMemcpyHostToDevice, s));
-    Grid G{d_data, d_mask, hd.m_data_shape[0], hd.m_data_shape[1], hd.m_data_shape[2], hd.m_mask_shape[0],
-           hd.m_mask_shape[1], hd.m_mask_shape[2], hd.m_data_strides[0], hd.m_data_strides[1],
-           hd.m_data_strides[2], hd.m_mask_strides[0], hd.m_mask_strides[1], hd.m_mask_strides[2]};
+    // A mask larger than the data: only its cells that have data count.
+    Grid G{d_data, d_mask, hd.m_data_shape[0], hd.m_data_shape[1], hd.m_data_shape[2], hd.m_data_strides[0],
+           hd.m_data_strides[1], hd.m_data_strides[2], hd.m_mask_strides[0], hd.m_mask_strides[1],
+           hd.m_mask_strides[2]};
     // informed cells: bit rows of the mask, and the walked words with any
-    const int wxm = (G.mx + 31) / 32, wx = (G.nx + 31) / 32, pad = (reach + 31) / 32;
-    const int wpr = wxm + 2 * pad + 1;
-    const long long mrows = (long long)G.my * G.mz, nall = mrows * wxm, nwalk = (long long)G.ny * G.nz * wx;
-    unsigned *d_bits = M.alloc<unsigned>((size_t)(mrows * wpr));
-    CV_CHECK(cudaMemsetAsync(d_bits, 0, (size_t)(mrows * wpr) * 4, s));
-    k_cv_bits<<<(unsigned)((nall * 32 + NT - 1) / NT), NT, 0, s>>>(G, wxm, wpr, pad, nall, d_bits);
+    const int wx = (G.nx + 31) / 32, pad = (reach + 31) / 32;
+    const int wpr = wx + 2 * pad + 1;
+    const long long rows = (long long)G.ny * G.nz, nwalk = rows * wx;
+    unsigned *d_bits = M.alloc<unsigned>((size_t)(rows * wpr));
+    CV_CHECK(cudaMemsetAsync(d_bits, 0, (size_t)(rows * wpr) * 4, s));
+    k_cv_bits<<<(unsigned)((nwalk * 32 + NT - 1) / NT), NT, 0, s>>>(G, wx, wpr, pad, nwalk, d_bits);
     const long long nb = (nwalk + NT - 1) / NT;
     long long *d_bc = M.alloc<long long>((size_t)nb);
     long long *d_tot = M.alloc<long long>(2);  // words with informed cells, informed cells

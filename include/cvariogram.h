@@ -71,6 +71,8 @@ void fill_ellipsoid_directions(struct ellipsoid_t *ell, double azimuth, double d
    every lag whose window holds the offset's length; a lag without pairs is
    NaN (0/0), as in the reference.  percentToUse < 100 keeps that share of the
    pairs, chosen by a hash of (offset, cell) -- the reference draws rand().
+   The mask may be larger than the data; its cells outside the data's shape do
+   not count (the reference reads past the data for them).
    On the GPU; per-lag pair counts exact, sums exact to 2^-100 relative. */
 void calc_variograms(struct variogram_search_template_t *templ, struct hard_data_t *data,
                      float *result_covariations, int result_length, int percentToUse);

@@ -42,3 +42,27 @@ def test_empty_mask(CV):  # noqa: F811
     v, m = VC.grid((40, 6, 2), 0.0, seed=4)
     sums, counts = CV.CalcVariogramStats(gpu_template(CV, VC.TEMPLATES["x_narrow"]), hard_data=(v, m))
     assert not sums.any() and not counts.any()
+
+
+@pytest.mark.parametrize("outside", [0, 1])
+def test_mask_larger_than_the_data(CV, outside):  # noqa: F811
+    """The mask's cells outside the data's shape do not count, informed or not."""
+    for shape, wider in (((31, 6, 3), (40, 6, 3)), ((33, 5, 4), (70, 9, 6)), ((64, 4, 2), (64, 5, 2))):
+        v, m = VC.grid(shape, 0.6, seed=shape[0])
+        big = np.full(wider, outside, np.uint8, order="F")
+        big[tuple(slice(n) for n in shape)] = m
+        for name in ("x_narrow", "overlapping_lags", "dipping"):
+            for percent in (100, 40):
+                t = gpu_template(CV, VC.TEMPLATES[name])
+                got = CV.CalcVariogramStats(t, hard_data=(v, big), percent=percent)
+                if percent == 100:
+                    o = O.variograms(O.cv_template(*VC.TEMPLATES[name]), v, m)
+                    assert np.array_equal(got[1], o["counts"]) and np.array_equal(got[0], o["exact_sums"])
+                else:
+                    # the sample is drawn by the mask's cell index
+                    big0 = big.copy("F")
+                    big0[shape[0]:] = 0
+                    big0[:, shape[1]:] = 0
+                    big0[:, :, shape[2]:] = 0
+                    want = CV.CalcVariogramStats(t, hard_data=(v, big0), percent=percent)
+                    assert np.array_equal(got[1], want[1]) and np.array_equal(got[0], want[0])
