@@ -9,7 +9,11 @@
 // so no field borrows from the next, and a field's top bit is set in both
 // exactly when -T <= v <= T.  Three comparisons of three differences become
 // one of the whole word.  m (the top bits) is 0 when the fields need more
-// than 32 bits: extents of several hundred cells on all three axes.
+// than 32 bits together: a field has two bits more than the largest power of
+// two in reach + T.  The models that are cut at the search radii (T = the
+// radii) pack up to several hundred cells on every axis; ordinary kriging and
+// cokriging, whose T is about the reach, up to 256 cells on every axis, or more
+// on one and fewer on the others, when the search spans them.
 #pragma once
 
 #ifdef __CUDACC__
