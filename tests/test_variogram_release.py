@@ -1,6 +1,7 @@
 """The device memory that variogram calls keep for the next one: bounded, and
-given back on request.  In a process of its own, so that nothing else moves the
-device's free memory."""
+given back on request.  In a process of its own, so that little else moves the
+device's free memory: the driver's own pages for the process still do, 64 kB at
+a time, while a pool takes and returns memory in units of UNIT bytes."""
 
 import os
 import subprocess
@@ -9,6 +10,7 @@ import sys
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+UNIT = 2 << 20  # the granularity of device allocations (cuMemGetAllocationGranularity)
 
 CHILD = """
 import ctypes as C
@@ -48,6 +50,6 @@ def test_kept_memory(native_lib):
                        env=dict(os.environ, PYTHONPATH=ROOT))
     assert r.returncode == 0, r.stderr
     kept, after, kept_huge, end = (int(x) for x in r.stdout.split())
-    assert kept > 0 and after == 0 and end == 0, r.stdout
+    assert kept >= UNIT and after < UNIT and end < UNIT, r.stdout
     # 256 MB stay, and what the device rounds an allocation up to
     assert kept_huge <= (256 << 20) + (64 << 20), r.stdout
