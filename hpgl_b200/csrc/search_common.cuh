@@ -86,37 +86,6 @@ __device__ __forceinline__ int template_segment(const DevJob &J, const DevPlan &
     return base;
 }
 
-// neighbour_lookup_t::find (sugarbox_neighbour_lookup.h:35-61) for one node:
-// the warp tests 32 template entries at a time against the informed-bit rows
-// (lane t entry base + t, lanes in template order) and keeps the first
-// max_neighbours hits.  List and count go to J.nb / J.nbcount.
-__device__ __forceinline__ void template_node(const DevJob &J, const DevPlan &P, int node, int lane) {
-    int x, y, z;
-    node_xyz(J, node, x, y, z);
-    const int nmax = P.nmax;
-    int *out = J.nb + (long long)node * nmax;
-    int cnt = 0;
-    for (int tb = 0; tb < P.tmpl_len && cnt < nmax; tb += 32) {
-        const int t = tb + lane;
-        bool hit = false;
-        int delta = 0;
-        if (t < P.tmpl_len) {
-            const int4 e = __ldg(&P.tmpl[t]);
-            delta = e.w;
-            const int yy = y + e.y, zz = z + e.z;
-            if ((unsigned)yy < (unsigned)J.ny && (unsigned)zz < (unsigned)J.nz) {
-                const int px = x + e.x;  // padded x of the target cell
-                hit = (J.bits[((long long)zz * J.ny + yy) * P.wpr + (px >> 5)] >> (px & 31)) & 1u;
-            }
-        }
-        const unsigned b = __ballot_sync(FULL_MASK, hit);
-        const int rank = __popc(b & ((1u << lane) - 1u));
-        if (hit && cnt + rank < nmax) out[cnt + rank] = node + delta;
-        cnt += __popc(b);
-    }
-    if (lane == 0) J.nbcount[node] = min(cnt, nmax);
-}
-
 // One lane's template entry of a speculative search: the informed and
 // pending words of its target cell, loaded ahead of their use.
 struct SpecProbe {
@@ -142,10 +111,12 @@ __device__ __forceinline__ SpecProbe spec_probe(const DevJob &J, const DevPlan &
     return q;
 }
 
-// neighbour_lookup_t::find for one node of a speculative simulation round
-// (path rank `rank`): as template_node, over the committed nodes of lower
-// rank (informed bit set and rank_of below `rank`; informed data have rank
-// -1); the list goes to `out`, its length to `count`.  Returns -1 when the
+// neighbour_lookup_t::find (sugarbox_neighbour_lookup.h:35-61) for one node of
+// a speculative simulation round (path rank `rank`): the warp tests 32 template
+// entries at a time against the informed-bit rows (lane t entry base + t) and
+// keeps, in template order, the first max_neighbours committed nodes of lower
+// rank (informed bit set and rank_of below `rank`; informed data have rank -1);
+// the list goes to `out`, its length to `count`.  Returns -1 when the
 // search completed, else the rank of the first pending node of lower rank met
 // before the point where the search would stop: in the sequential order that
 // node would have been simulated and seen, so nothing of this search is kept.
