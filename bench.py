@@ -380,7 +380,7 @@ def main():
             "fp64": {"value": fp64_value, "ms_per_step": t_fp64 / args.steps,
                      "top_kernel_ms": info_f["ms_top_kernel"]},
             "mixed_vs_fp64": value / fp64_value,
-            "routed_to_fp64": info_m["systems_fp64"] / max(1, info_m["systems"]),
+            "share_fp64": info_m["systems_fp64"] / max(1, info_m["systems"]),
             "e2e": {"value": e2e["mixed"]["value"], "unit": "nodes/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "ms_per_step": e2e["mixed"]["ms_per_step"],
                     "split_ms": e2e["mixed"]["split_ms"],

@@ -27,7 +27,7 @@ def _case(name, job, kind, N, steps, warmup):
                           "top_kernel": info["top_kernel"], "ms_top_kernel": info["ms_top_kernel"]}
         if precision == "mixed":
             out["systems"] = int(systems)
-            out["rerouted_to_fp64"] = (info["systems_fp64"] / systems) if systems else 0.0
+            out["share_fp64"] = (info["systems_fp64"] / systems) if systems else 0.0
     # whole calls from host buffers: one warm-up (first-use costs: pinned
     # staging, arena growth, module loading), then the median of three
     N.krige(job, precision="mixed", kind=kind)

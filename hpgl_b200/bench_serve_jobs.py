@@ -51,7 +51,7 @@ def run(args, root):
             ms, info = N.bench(job, precision=precision, iters=steps, warmup=warmup, flush_bytes=0)
             row[precision] = {"ms": float(np.median(ms)), "ms_search": info["ms_search"],
                               "top_kernel": info["top_kernel"], "ms_top_kernel": info["ms_top_kernel"],
-                              "ms_resolve": info["ms_resolve"], "systems": int(info["systems"]),
+                              "systems": int(info["systems"]),
                               "share_fp64": (info["systems_fp64"] / info["systems"]) if info["systems"] else 0.0}
         rows.append(row)
         print(json.dumps(row), flush=True)

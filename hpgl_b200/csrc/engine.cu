@@ -526,9 +526,9 @@ static DevJob make_devjob(const JobState &S, const Group &g) {
 }
 
 // Events around the first group's phases: search start, solve start, solve
-// end (top kernel), re-solve end.
+// end (top kernel).
 struct PassTiming {
-    cudaEvent_t search0 = nullptr, top0 = nullptr, top1 = nullptr, resolve1 = nullptr;
+    cudaEvent_t search0 = nullptr, top0 = nullptr, top1 = nullptr;
     int launches = 0;
 };
 
@@ -557,10 +557,7 @@ static void device_pass(JobState &S, cudaStream_t s, PassTiming *pt,
             CUDA_CHECK(cudaMemsetAsync(J.node_next, 0, sizeof(int), s));
             if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top0, s));
             launch_cokriging(J, g.dp, s);
-            if (pt && gi == 0) {
-                CUDA_CHECK(cudaEventRecord(pt->top1, s));
-                CUDA_CHECK(cudaEventRecord(pt->resolve1, s));
-            }
+            if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top1, s));
             launches += 2;
             CUDA_CHECK(cudaGetLastError());
             if (after_group) after_group(g);
@@ -586,7 +583,6 @@ static void device_pass(JobState &S, cudaStream_t s, PassTiming *pt,
         }
         ++launches;
         if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top1, s));
-        if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->resolve1, s));
         CUDA_CHECK(cudaGetLastError());
         if (after_group) after_group(g);
     }
@@ -1113,13 +1109,12 @@ void bench_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res, hpgl_b200_be
     CUDA_CHECK(cudaEventCreate(&pt.search0));
     CUDA_CHECK(cudaEventCreate(&pt.top0));
     CUDA_CHECK(cudaEventCreate(&pt.top1));
-    CUDA_CHECK(cudaEventCreate(&pt.resolve1));
     cudaEvent_t e0, e1;
     CUDA_CHECK(cudaEventCreate(&e0));
     CUDA_CHECK(cudaEventCreate(&e1));
     // Phase times from eager passes (events between the launches), then the
     // timed iterations as graph replays.
-    double top_sum = 0, search_sum = 0, resolve_sum = 0;
+    double top_sum = 0, search_sum = 0;
     const int phase_runs = std::max(1, std::min(bench.iters, 3));
     for (int it = 0; it < 1 + phase_runs; ++it) {
         if (bench.flush_bytes > 0)
@@ -1127,13 +1122,11 @@ void bench_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res, hpgl_b200_be
         device_pass(S, C.stream, &pt, nullptr);
         read_counters(S, C.stream);
         if (it == 0) continue;  // first use of every kernel
-        float tms = 0, sms = 0, rms = 0;
+        float tms = 0, sms = 0;
         cudaEventElapsedTime(&tms, pt.top0, pt.top1);
         cudaEventElapsedTime(&sms, pt.search0, pt.top0);
-        cudaEventElapsedTime(&rms, pt.top1, pt.resolve1);
         top_sum += tms;
         search_sum += sms;
-        resolve_sum += rms;
     }
     PassGraph G;
     capture_pass(S, C.stream, G);
@@ -1153,13 +1146,12 @@ void bench_job(const hpgl_b200_job_t &job, hpgl_b200_result_t &res, hpgl_b200_be
     }
     bench.ms_top_kernel = top_sum / phase_runs;
     bench.ms_search = search_sum / phase_runs;
-    bench.ms_resolve = resolve_sum / phase_runs;
+    bench.ms_resolve = 0;
     snprintf(bench.top_kernel, sizeof(bench.top_kernel), "%s", top_kernel_name(S));
     bench.launches_per_iter = pt.launches;
     cudaEventDestroy(pt.search0);
     cudaEventDestroy(pt.top0);
     cudaEventDestroy(pt.top1);
-    cudaEventDestroy(pt.resolve1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     download(S, res, cnt, C.stream);

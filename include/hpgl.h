@@ -386,7 +386,7 @@ typedef struct hpgl_b200_bench_t {
     long long systems_fp64;
     double ms_plan;
     double ms_search;             /* average device time of the first group's searches */
-    double ms_resolve;            /* ... and of what follows its solve (nothing in this build) */
+    double ms_resolve;            /* 0: nothing follows the solves in this build */
 } hpgl_b200_bench_t;
 int hpgl_b200_bench(const hpgl_b200_job_t *job, hpgl_b200_result_t *result, hpgl_b200_bench_t *bench);
 
