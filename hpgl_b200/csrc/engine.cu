@@ -558,7 +558,7 @@ static void device_pass(JobState &S, cudaStream_t s, PassTiming *pt,
             if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top0, s));
             launch_cokriging(J, g.dp, s);
             if (pt && gi == 0) CUDA_CHECK(cudaEventRecord(pt->top1, s));
-            launches += 2;
+            launches += cok_tile_takes(g.dp) ? 3 : 2;  // the tiles and the marked nodes' kernel
             CUDA_CHECK(cudaGetLastError());
             if (after_group) after_group(g);
             continue;
