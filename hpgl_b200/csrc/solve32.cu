@@ -669,6 +669,12 @@ __global__ void __launch_bounds__(256) k_sis_draw(DevJob J, SgsState G, int cur)
     }
 }
 
+// A simulation's systems take every other of the solve's tiles (launch_solve32):
+// a round's solve is the smaller part of it beside the search, and 24 in place
+// of 20 and 32 in place of 28 cost SGS 166x141x100 20.24 for 19.47 ms and 30.5
+// for 29.5.  Above 32 neighbours search and system stay in one warp
+// (launch_sgs_try64), 131 ms at 40 and 218 at 64 there; the tiles of up to 64
+// in a trial build took 48 and 114.
 bool sim_tiles(const DevPlan &P) { return P.nmax <= 32 && tile_takes(P); }
 
 void launch_sis_groups(const DevJob &J, const SisGroups &groups, const SgsState &G, int cur, cudaStream_t s) {
@@ -727,8 +733,13 @@ void launch_fused32(const DevJob &J, const DevPlan &P, cudaStream_t s, int block
 // system share each step's pivot chain among more systems and read fewer
 // shared-memory words per product, until the lane's accumulators no longer
 // fit the registers: 4 lanes (8 systems a warp) up to 24 neighbours, 8 above;
-// the panel (row blocks whose sums are kept open together) is the widest
-// that does not spill.  Solve of the IK 200x200x100 job (4.0 M systems) with
+// the panel (row blocks whose sums are kept open together) trades spilled
+// registers, which every width has some of, for passes over the finished rows.
+// Panels of another width on SK 256x256x64 with the neighbour count set, in ms
+// (panel taken [width: ms]): 12: 2.01 [2: 1.95]   16: 3.20 [4: 3.28]   20: 7.25
+// [4: 6.42]   24: 9.84 [4: 9.33]   28: 14.8 [2: 17.0, 6: 15.4]   32: 17.4 [2:
+// 17.6, 6: 18.6]; up to 24 the other width spills more (24: 300 bytes for 24)
+// and is the faster one at 12, 20 and 24 all the same.  Solve of the IK 200x200x100 job (4.0 M systems) with
 // the neighbour count set, in ms:
 //   8: 1.06   12: 1.99   16: 3.09   20: 7.1   24: 9.1   28: 14.5
 // against 39.7 at 24 with one column per lane and one system a warp; SK

@@ -671,7 +671,11 @@ __global__ void __launch_bounds__(WARPS64_BLOCK * 32) k_sis_try64(DevJob J, cons
 // a warp, two columns a lane): 36: 28.8   40: 34.0 [149.6]   44: 40.7   48:
 // 45.1 [181.7]   52: 66.2   56: 76.3 [211.3]   64: 106.1 [241.7], 123.2 with
 // 16 lanes; LVM 512x512x32 (7.5 M systems, 64) 175.7 [327], with 16
-// lanes 244.
+// lanes 244.  Panels (row blocks whose sums are kept open together) two blocks
+// narrower / wider on the same job: 36: 28.4 / 29.4   40: 33.1 / 34.6   44: 40.6
+// / 41.3   48: 45.6 / 48.7   52: 70.5 / 71.3   56: 78.5 / 78.8   64: 111.7 / 109.5;
+// at 36 and 40, where the panel of 4 spills 120 and 184 bytes, the narrower one
+// would be 2 % faster.
 void launch_solve64(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
     const int b = blocks_per_sm;
     if (!tile_takes(P)) {

@@ -5,8 +5,8 @@
 //
 // Measured on SK 256x256x64 (4.15 M systems of 32 neighbours): 17.5 ms where
 // one column per lane and one system a warp took 53.2 ms.  ncu on the
-// 128x128x32 cube: 2 300 instructions a system (8 387), FP64 pipe 30 %, the
-// shared-memory / L1 data pipe 58 %, 8 warps an SM (their registers hold the
+// 128x128x32 cube: 2 251 instructions a system (8 387), FP64 pipe 31.8 %, the
+// shared-memory / L1 data pipe 61.5 %, 8 warps an SM (their registers hold the
 // accumulators): the pivot chain's latency and the L1 pipe bound it now.
 //
 // What bounds a small Cholesky factorisation is not its arithmetic: every
