@@ -437,10 +437,14 @@ static void upload_rest(JobState &S, cudaStream_t s) {
         d.syx = d.sx * (2 * P.B[1] + 1);
         d.truncated = P.truncated ? 1 : 0;
         {
-            // offsets reach the radii (template) or 2 r - 1 (clusterizer boxes)
+            // two neighbours' offsets differ by at most what the table of an
+            // untruncated model is sized for (build_plan)
             const int n3[3] = {P.nx, P.ny, P.nz}, t3[3] = {d.Tx, d.Ty, d.Tz};
             int reach[3];
-            for (int a = 0; a < 3; ++a) reach[a] = (int)std::min<long long>(n3[a] - 1, 4LL * P.radii[a]);
+            for (int a = 0; a < 3; ++a) {
+                const long long pairs = std::max(2LL * P.ext[a], P.any_clean ? 4LL * P.radii[a] - 2 : 0LL);
+                reach[a] = (int)std::min<long long>(n3[a] - 1, pairs);
+            }
             d.pk = OffsetPack(reach, t3);
         }
         d.c0 = P.c0;

@@ -149,13 +149,12 @@ inline int tuning_family(int nmax) { return nmax <= 32 ? 0 : 1; }
 long long persistent_grid(const void *fn, int threads, size_t smem, int blocks_per_sm, long long units);
 
 // The jobs the tiled kernels take: neighbour offsets that pack into one word
-// (OffsetPack: extents and ranges whose fields need at most 32 bits together)
-// and a sill whose pivots stay in sqrt_rcp's range.  The others keep the
+// (OffsetPack) and a sill whose pivots stay in sqrt_rcp's range.  The others keep the
 // one-system-a-warp kernels.
 constexpr double PIVOT_C0_MIN = 0x1p-600, PIVOT_C0_MAX = 0x1p+700;
-inline bool tile_takes(const DevPlan &P) { return P.pk.m != 0 && P.c0 >= PIVOT_C0_MIN && P.c0 < PIVOT_C0_MAX; }
+inline bool tile_takes(const DevPlan &P) { return P.pk.fits && P.c0 >= PIVOT_C0_MIN && P.c0 < PIVOT_C0_MAX; }
 // ... and the tiled cokriging, whose square fits a warp's registers up to 48.
-inline bool cok_tile_takes(const DevPlan &P) { return P.pk.m != 0 && P.nmax <= 48; }
+inline bool cok_tile_takes(const DevPlan &P) { return P.pk.fits && P.nmax <= 48; }
 
 // Launchers (stream-ordered, no synchronisation).
 void launch_build_bits(const DevJob &J, const DevPlan &P, uint32_t *bits, cudaStream_t s);
