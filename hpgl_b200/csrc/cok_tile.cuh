@@ -261,9 +261,9 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_cok_tile(DevJob J, DevPlan
                 int k = 0;
                 if (lane == 0) k = atomicAdd(J.node_next, csize);
                 base = __shfl_sync(FULL_MASK, k, 0);
-                more = base >= 0 && base < J.size;
-                const int i = base + lane;
-                bool solve = more && lane < csize && i < J.size;
+                more = chunk_first(base, J.size) < J.size;
+                const int i = (int)((unsigned)base + (unsigned)lane);
+                bool solve = more && chunk_has(base, lane, csize, J.size);
                 if (solve && J.mask[i]) {
                     // informed primary: copied (set_at, simple_cokriging_markI.cpp:245-248)
                     J.out_values[i] = J.values[i];

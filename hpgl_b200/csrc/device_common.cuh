@@ -3,6 +3,7 @@
 #include <cstdint>
 
 #include "kernels.cuh"
+#include "node_chunk.h"
 
 namespace hpgl_b200 {
 

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256) k_search_template(DevJob J, DevPlan P) {
         int segi = 0;
         if (lane == 0) segi = atomicAdd(J.seg_next, 1);
         segi = __shfl_sync(FULL_MASK, segi, 0);
-        if (segi >= total) break;
+        if (chunk_first(segi, total) >= total) break;
         template_segment(J, P, segi, lane, delta_sm[wib]);
     }
 }
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(CLUSTER_WARPS * 32, 16) k_search_cluster(DevJo
         int chunk = 0;
         if (lane == 0) chunk = atomicAdd(J.node_next, take);
         chunk = __shfl_sync(FULL_MASK, chunk, 0);
-        if (chunk >= J.size) break;
+        if (chunk_first(chunk, J.size) >= J.size) break;
         const int chunk_end = (int)min((long long)chunk + take, (long long)J.size);
         for (int node = chunk; node < chunk_end; ++node) {
             if (!node_needs_kriging(J, node)) continue;

@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(WARPS32 * 32) k_solve_exact32(DevJob J, DevPla
     int chunk = 0;
     if (lane == 0) chunk = atomicAdd(J.node_next, csize);
     chunk = __shfl_sync(FULL_MASK, chunk, 0);
-    long long it = chunk;
+    long long it = chunk_first(chunk, J.size);
     NodeFetch cur = fetch_node(J, P, it < J.size ? (int)it : -1, lane);
     while (it < J.size) {
         long long nx = it + 1;
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(WARPS32 * 32) k_solve_exact32(DevJob J, DevPla
             int c = 0;
             if (lane == 0) c = atomicAdd(J.node_next, csize);
             nchunk = __shfl_sync(FULL_MASK, c, 0);
-            nx = nchunk;
+            nx = chunk_first(nchunk, J.size);
         }
         const NodeFetch next = fetch_node(J, P, nx < J.size ? (int)nx : -1, lane);
         solved += exact32_node(J, P, S, cur, lane);
@@ -737,8 +737,8 @@ void launch_fused32(const DevJob &J, const DevPlan &P, cudaStream_t s, int block
 // registers, which every width has some of, for passes over the finished rows.
 // Panels of another width on SK 256x256x64 with the neighbour count set, in ms
 // (panel taken [width: ms]): 12: 2.01 [2: 1.95]   16: 3.20 [4: 3.28]   20: 7.25
-// [4: 6.42]   24: 9.84 [4: 9.33]   28: 14.8 [2: 17.0, 6: 15.4]   32: 17.4 [2:
-// 17.6, 6: 18.6]; up to 24 the other width spills more (24: 300 bytes for 24)
+// [4: 6.42]   24: 9.65 [4: 9.33]   28: 14.8 [2: 17.0, 6: 15.4]   32: 17.4 [2:
+// 17.6, 6: 18.6]; up to 24 the other width spills more (24: 300 bytes for 8)
 // and is the faster one at 12, 20 and 24 all the same.  Solve of the IK 200x200x100 job (4.0 M systems) with
 // the neighbour count set, in ms:
 //   8: 1.06   12: 1.99   16: 3.09   20: 7.1   24: 9.1   28: 14.5

@@ -514,14 +514,14 @@ __global__ void __launch_bounds__(WARPS64_BLOCK * 32) k_solve_exact64(DevJob J, 
     // solved), so none waits on a fixed share at the end
     const int csize = chunk_nodes(J, CHUNK64, WARPS64_BLOCK);
     int chunk = take_chunk64(J, lane, csize);
-    long long it = chunk;
+    long long it = chunk_first(chunk, J.size);
     NodeFetch cur = fetch_node(J, P, it < J.size ? (int)it : -1, lane);
     while (it < J.size) {
         long long nx = it + 1;
         int nchunk = chunk;
         if (nx == (long long)chunk + csize) {
             nchunk = take_chunk64(J, lane, csize);
-            nx = nchunk;
+            nx = chunk_first(nchunk, J.size);
         }
         const NodeFetch next = fetch_node(J, P, nx < J.size ? (int)nx : -1, lane);
         solved += exact64_node(J, P, S, s_cs, cur, lane);
@@ -668,13 +668,13 @@ __global__ void __launch_bounds__(WARPS64_BLOCK * 32) k_sis_try64(DevJob J, cons
 // than the better occupancy gives: issue slots in use 48 % for 31 %.  At 56
 // and below they cost more (56: 85.2, 48: 61.0, 40: 43.8 ms).  Solve of SK
 // 256x256x64 (4.15 M systems) with the neighbour count set, in ms (one system
-// a warp, two columns a lane): 36: 28.8   40: 34.0 [149.6]   44: 40.7   48:
+// a warp, two columns a lane): 36: 28.8   40: 34.0 [149.6]   44: 39.1   48:
 // 45.1 [181.7]   52: 66.2   56: 76.3 [211.3]   64: 106.1 [241.7], 123.2 with
 // 16 lanes; LVM 512x512x32 (7.5 M systems, 64) 175.7 [327], with 16
 // lanes 244.  Panels (row blocks whose sums are kept open together) two blocks
 // narrower / wider on the same job: 36: 28.4 / 29.4   40: 33.1 / 34.6   44: 40.6
 // / 41.3   48: 45.6 / 48.7   52: 70.5 / 71.3   56: 78.5 / 78.8   64: 111.7 / 109.5;
-// at 36 and 40, where the panel of 4 spills 120 and 184 bytes, the narrower one
+// at 36 and 40, where the panel of 4 spills 120 and 196 bytes, the narrower one
 // would be 2 % faster.
 void launch_solve64(const DevJob &J, const DevPlan &P, cudaStream_t s, int blocks_per_sm) {
     const int b = blocks_per_sm;

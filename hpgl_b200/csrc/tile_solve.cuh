@@ -573,9 +573,9 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_solve_tile(DevJob J, DevPl
                 int c = 0;
                 if (lane == 0) c = atomicAdd(J.node_next, csize);
                 base = __shfl_sync(FULL_MASK, c, 0);
-                more = base >= 0 && base < J.size;
-                const int i = base + lane;
-                bool solve = more && lane < csize && i < J.size;
+                more = chunk_first(base, J.size) < J.size;
+                const int i = (int)((unsigned)base + (unsigned)lane);
+                bool solve = more && chunk_has(base, lane, csize, J.size);
                 if (solve && is_cont(J.kind) && J.mask[i] != 0) {
                     J.out_values[i] = J.values[i];
                     J.out_mask[i] = 1;
